@@ -50,7 +50,6 @@ cudaError_t launch_wy_apply(const WyArgs& a, int batch, cudaStream_t st);
 // its own array (rows 0..N-1), with block columns 0..L-2 at A; without them
 // it is A's block column L-1.
 int bsof_leaf_width(int n);
-void bsof_set_factor_warps(int w);
 // TMA loading of the persistent BSOI's clean 128 x 128 tiles; process-wide.
 void bsoi_set_tma(int on);
 int bsof_tiles(int n);

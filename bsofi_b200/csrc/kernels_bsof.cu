@@ -4,7 +4,7 @@
 // the stacked 2n x n panel [R~_k; B_k] at A_BLK(k,k), dormqr('L','T') of
 // A_BLK(k,k+1) and A_BLK(k,L-1); then dgeqrf of the final 2n x 2n block.
 //
-// Work decomposition.  Every block column is cut into tiles of NB columns
+// Work decomposition.  Every block column is cut into tiles of 16 columns
 // (the last one may be narrower).  A "leaf" is the Householder QR of one tile
 // inside its panel; leaves are numbered s = 0..S-1 in the reference's order
 // (panel k, left to right; the final panel has the tiles of block columns L-2
@@ -23,810 +23,1019 @@
 // only on tasks earlier in that order and all CTAs are co-resident
 // (cooperative launch), so the schedule cannot deadlock; every spin is
 // bounded and sets an error word instead of hanging.
-#include <atomic>
+//
+// The chain is a serial sequence of N Householder columns, so its time is the
+// latency of one column step.  The leaf stays in registers from one leaf to
+// the next, laid out as the accumulators of mma.m16n8k8.f64 hold C^T: lane
+// 4 g + t of a warp owns two columns and rows 2t, 2t+1 of each of its 8-row
+// blocks.  That layout makes a column step cheap in every part: the pivot
+// column reaches the lanes of a row block by one shuffle per row, a column's
+// dot products end in a sum over four lanes (a DMMA with ones), and there is
+// one barrier per column, after which every warp sums the warps' partials and
+// forms the reflector's scalars for itself (a second barrier, with one warp
+// forming them for all, measured the same at n = 256 and slower below; two
+// columns per barrier, the second one's products corrected for the first
+// reflector, measured slower everywhere: one warp's scalar code then takes
+// longer than the barrier it saves).  The 16 pivot rows of a leaf belong to
+// one warp of their own (the top warp), so the row warps need no row masks; T
+// is built one column behind by another.  The same registers are the B operand
+// of W^T = C^T V and the accumulators of C^T -= (W T)^T V^T, so the update of
+// the next tile reads V from shared memory once and leaves the tile where the
+// next factorization wants it.
+//
+// Measured (chain of one inversion, ms; before: two barriers a column, a
+// five-level shuffle sum of 16 values a thread, the tile through L2 and shared
+// memory between leaves, 8-wide leaves above n = 256): n = 64, p = 16 1.03 ->
+// 0.55; n = 100, p = 64 6.87 -> 4.63; n = 256, p = 32 10.6 -> 7.1; n = 400,
+// p = 64 41.2 -> 32.  Per 16-column leaf at n = 256: 9.5 us of column steps
+// (about 1160 cycles each, half of them FP64 issue: DFMA takes 3 cycles a warp
+// instruction per scheduler), 1.2 us for each half of the next tile's update
+// (64 cycles per m16n8k8, two row warps per scheduler).
 #include <climits>
-#include "bsofi_common.cuh"
+#include <type_traits>
+#include "bsof_sched.cuh"
 #include "bsofi_kernels.h"
+#include "tcgen05.cuh"
 
 namespace bsofi {
 
-constexpr int BT = 256;  // threads per CTA
-constexpr int BW = BT / 32;
-
-struct BsofGeom {
-  int n, L, NB, nl, S;
-  int form_g;  // 1: leaves also update G_k = Q_k^T (identity-initialised by the caller)
+// FW row warps of NI 8-row blocks each, one top warp, helper warps.  PREF:
+// the next tile fits in shared memory beside V and is staged there by the
+// helper warps while the leaf is factored.  NIW: 8-row blocks per warp of a
+// worker (all FW + 1 warps take rows there).
+template <int FW_, int NI_, int NIW_, bool PREF_>
+struct ChainCfg {
+  static constexpr int FW = FW_, NI = NI_, NIW = NIW_;
+  static constexpr bool PREF = PREF_;
+  static constexpr int MW = FW + 1, MT = 32 * MW;
+  static constexpr int HW = 4;
+  static constexpr int THREADS = MT + 32 * HW;
+  static constexpr int CT = MT + 32;  // column barrier: with the T warp, the last helper
+  // Row slots are taken in groups of GS, skipped when every row is finished.
+  static constexpr int GS = 3, NG = (NI + GS - 1) / GS;
+  // The pivot column's shuffled values are kept from the dot products to the
+  // update where registers allow, else shuffled again.
+  static constexpr bool KEEPX = NI <= 14;
+  // Tiles move between global and shared memory by bulk copies, which keep the
+  // load/store pipe free for the computing warps, or (short panels, where the
+  // chain waits for the workers' answer and latency counts) by cp.async and
+  // by stores of the warps that hold the reflectors.
+  static constexpr bool BULK = NI > 5;
+  // V as the operand of W = V^T C comes from the registers that factored it,
+  // or, where V and C do not fit in registers together, from shared memory.
+  static constexpr bool VREG = NI <= 9;
+  // With 12 warps a thread gets 168 registers at launch; the helper warpgroup
+  // gives most of its own to the two that compute
+  // (2 x 128 x 224 + 128 x 56 = 384 x 168).
+  static constexpr bool REGS = THREADS == 384;
+  // Largest panel height 2n: rows owned by the chain's warps and a worker's.
+  static constexpr int ROWS_CHAIN = 8 * (2 + FW * NI), ROWS_WORK = 8 * MW * NIW;
+  static constexpr int MAX_ROWS = ROWS_CHAIN < ROWS_WORK ? ROWS_CHAIN : ROWS_WORK;
+  static_assert(MW == 4 || MW == 8, "partial sums are read as 4 or 8 per column");
 };
 
-// Leaf s -> panel k, leaf index l in the panel, tile (m, t), panel column j0.
-struct Leaf {
-  int k, l, m, t, j0, w;
-};
-
-BSOFI_DEVINL Leaf leaf_of(const BsofGeom& g, int s) {
+// Leaf s as the chain CTA sees it.  Rows are counted from the top of the
+// panel, except in the second half of the final panel when n is not a
+// multiple of 16: there from its row n on, so that a leaf's first row is
+// always a multiple of 16.
+struct ChainStep {
   Leaf f;
-  const int reg = (g.L - 2) * g.nl;
-  if (s < reg) {
-    f.k = s / g.nl;
-    f.l = s % g.nl;
-    f.m = f.k;
-    f.t = f.l;
-    f.j0 = f.t * g.NB;
-  } else {
-    f.k = g.L - 2;
-    f.l = s - reg;
-    if (f.l < g.nl) {
-      f.m = g.L - 2;
-      f.t = f.l;
-      f.j0 = f.t * g.NB;
-    } else {
-      f.m = g.L - 1;
-      f.t = f.l - g.nl;
-      f.j0 = g.n + f.t * g.NB;
-    }
-  }
-  f.w = min(g.NB, g.n - f.t * g.NB);
-  return f;
-}
-
-BSOFI_DEVINL int tile_id(const BsofGeom& g, int m, int t) { return m * g.nl + t; }
-
-BSOFI_DEVINL void tile_range(const BsofGeom& g, int m, int t, int& lo, int& hi) {
-  if (m >= g.L) {  // G_k tile: every leaf of panel k, in order
-    const int k = (m - g.L) / 2;
-    lo = k * g.nl;
-    hi = lo + (k <= g.L - 3 ? g.nl : 2 * g.nl);
-    return;
-  }
-  if (m <= g.L - 2) {
-    lo = max(0, (m - 1) * g.nl);
-    hi = m * g.nl + t;
-  } else {
-    lo = 0;
-    hi = (g.L - 1) * g.nl + t;
-  }
-}
-
-// Number of targets of leaf s; target q (0 = tile of leaf s+1).  With
-// form_g the 2*nl column tiles of G_k follow the matrix targets; they are
-// reported as block columns m = L + 2k + h (h = 0, 1) of a virtual matrix.
-BSOFI_DEVINL int ntargets(const BsofGeom& g, const Leaf& f) {
-  const int gt = g.form_g ? 2 * g.nl : 0;
-  if (f.k <= g.L - 3) return (g.nl - 1 - f.l) + 2 * g.nl + gt;
-  return 2 * g.nl - 1 - f.l + gt;
-}
-
-BSOFI_DEVINL void target_of(const BsofGeom& g, const Leaf& f, int q, int& m, int& t) {
-  const int nmat = (f.k <= g.L - 3) ? (g.nl - 1 - f.l) + 2 * g.nl : 2 * g.nl - 1 - f.l;
-  if (q >= nmat) {
-    const int u = q - nmat;
-    m = g.L + 2 * f.k + u / g.nl;
-    t = u % g.nl;
-    return;
-  }
-  if (f.k <= g.L - 3) {
-    const int np = g.nl - 1 - f.l;
-    if (q < np) {
-      m = f.k;
-      t = f.l + 1 + q;
-    } else if (q < np + g.nl) {
-      m = f.k + 1;
-      t = q - np;
-    } else {
-      m = g.L - 1;
-      t = q - np - g.nl;
-    }
-  } else {
-    int u = f.l + 1 + q;
-    if (u < g.nl) {
-      m = g.L - 2;
-      t = u;
-    } else {
-      m = g.L - 1;
-      t = u - g.nl;
-    }
-  }
-}
-
-// Worker tasks before leaf s (each leaf contributes ntargets - 1 tasks).
-BSOFI_DEVINL long long tasks_before(const BsofGeom& g, int s) {
-  const int reg = (g.L - 2) * g.nl;
-  const long long nl = g.nl, gt = g.form_g ? 2 * nl : 0;
-  const long long per_reg_leaf0 = 3 * nl - 2 + gt;  // tasks of regular leaf l: 3nl - 2 - l + gt
-  const long long per_panel = nl * per_reg_leaf0 - nl * (nl - 1) / 2;
-  if (s <= reg) {
-    long long k = s / g.nl, l = s % g.nl;
-    return k * per_panel + l * per_reg_leaf0 - l * (l - 1) / 2;
-  }
-  long long base = (long long)(g.L - 2) * per_panel;
-  long long l = s - reg;  // final leaf l has max(2nl - 2 - l + gt, 0) tasks
-  if (gt > 0) return base + l * (2 * nl - 2 + gt) - l * (l - 1) / 2;
-  long long full = min(l, 2 * nl - 1);
-  return base + full * (2 * nl - 2) - full * (full - 1) / 2;
-}
-
-struct BsofState {
-  // Block columns 0..L-2 of the matrix at A (leading dimension ld), the last
-  // block column at Al (ldl).  The ordinary layout has Al = A + (L-1) n ld;
-  // the compact one stores block columns 0..L-2 with ld = 3n (every access
-  // of block column m stays in block rows m-1..m+1, so those windows never
-  // overlap) and the last block column as its own N x n array.
-  double* A;
-  long long ld;
-  double* Al;
-  long long ldl;
-  double* G;  // (L-1) x (2n)^2, used when form_g
-  double* tau;
-  double* T;  // 256 doubles per leaf: (k * maxleaves + l) * 256
-  int maxleaves;
-  int* cnt;       // per tile
-  int* factored;  // per leaf
-  int* next_task;
-  int* err;       // 0 ok; 1 timeout
-  long long spin_limit;
-  unsigned long long* timeline;  // 4 stamps per leaf from the panel CTA (diagnostics)
-  // This launch factors leaves [s_begin, s_end) and runs their worker tasks;
-  // the per-tile and per-leaf counters carry over from an earlier launch of
-  // the leaves before s_begin, whose updates are then all done.
-  int s_begin, s_end;
+  int base, ab, rows, nb;  // first row counted, the leaf's first row, panel rows, 8-row blocks
+  int m2, t2, lo2, w2;     // the tile of leaf s+1
+  bool next, fresh, trans;
+  double *P, *C;           // row 0, column 0 of the leaf's tile and of the next one
+  long long ldp, ldc;
 };
 
-// Element (row, column col of block column m) of the matrix, and the leading
-// dimension there.
-BSOFI_DEVINL double* mat_ptr(const BsofGeom& g, const BsofState& st, long long row, int m,
-                             int col, long long& ldm) {
-  if (m == g.L - 1) {
-    ldm = st.ldl;
-    return st.Al + cm(row, col, st.ldl);
+BSOFI_DEVINL int leaf_base(const BsofGeom& g, const Leaf& f) {
+  return (f.k == g.L - 2 && f.l >= g.nl && (g.n & 15) != 0) ? g.n : 0;
+}
+
+BSOFI_DEVINL ChainStep chain_step(const BsofGeom& g, const BsofState& st, int s) {
+  ChainStep c;
+  c.f = leaf_of(g, s);
+  c.base = leaf_base(g, c.f);
+  c.ab = c.f.j0 - c.base;
+  c.rows = 2 * g.n - c.base;
+  c.nb = (c.rows + 7) / 8;
+  c.next = ntargets(g, c.f) > 0;
+  c.m2 = c.t2 = c.lo2 = 0;
+  c.C = nullptr;
+  c.ldc = 2;
+  if (c.next) {
+    int hi2;
+    target_of(g, c.f, 0, c.m2, c.t2);
+    tile_range(g, c.m2, c.t2, c.lo2, hi2);
+    c.C = tile_ptr(g, st, c.f.k, c.base, c.m2, c.t2, c.ldc);
   }
-  ldm = st.ld;
-  return st.A + cm(row, (long long)m * g.n + col, st.ld);
+  c.P = mat_ptr(g, st, (long long)c.f.k * g.n + c.base, c.f.m, c.f.t * 16, c.ldp);
+  c.w2 = min(16, g.n - c.t2 * 16);
+  // Panel change (rows shift by n, n fresh rows come in), and the shift by n
+  // inside the final panel when n is not a multiple of 16.
+  c.fresh = c.next && c.f.l == g.nl - 1 && c.f.k <= g.L - 3;
+  c.trans = c.fresh || (c.next && c.f.l == g.nl - 1 && (g.n & 15) != 0);
+  return c;
 }
 
-// Column tile (m, t) of the matrix, or of G_k for m >= L: base pointer at the
-// leaf's first row j0 of its panel, and leading dimension.
-BSOFI_DEVINL double* tile_ptr(const BsofGeom& g, const BsofState& st, int k, int j0, int m, int t,
-                              long long& ldt) {
-  if (m >= g.L) {
-    const int kk = (m - g.L) / 2, h = (m - g.L) % 2;
-    const long long n2 = 2ll * g.n;
-    ldt = n2;
-    return st.G + (long long)kk * n2 * n2 + cm(j0, (long long)h * g.n + t * g.NB, n2);
-  }
-  return mat_ptr(g, st, (long long)k * g.n + j0, m, t * g.NB, ldt);
-}
-
-BSOFI_DEVINL unsigned long long gtimer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-
-BSOFI_DEVINL int ld_acquire(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-BSOFI_DEVINL void red_release_add(int* p, int v) {
-  asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Thread 0 waits until *p >= target (bounded); the result is broadcast.
-// Returns false when the wait timed out or another CTA reported an error.
-BSOFI_DEVINL bool block_wait_geq(const BsofState& st, const int* p, int target, int* sflag) {
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    long long it = 0;
-    while (ld_acquire(p) < target) {
-      if (ld_acquire(st.err) != 0) {
-        ok = 0;
-        break;
-      }
-      if (++it > st.spin_limit) {
-        atomicExch(st.err, 1);
-        ok = 0;
-        break;
-      }
-      __nanosleep(64);
-    }
-    *sflag = ok;
-  }
-  __syncthreads();
-  bool ok = *sflag != 0;
-  __syncthreads();
-  return ok;
-}
-
-// Barrier among the first `count` threads of the CTA (id 1; id 0 is __syncthreads).
-BSOFI_DEVINL void named_bar(int count) { asm volatile("bar.sync 1, %0;" ::"r"(count) : "memory"); }
-// Barrier id 2: the panel CTA's prefetch warps (concurrent with barrier 1).
-BSOFI_DEVINL void named_bar2(int count) { asm volatile("bar.sync 2, %0;" ::"r"(count) : "memory"); }
-
-// Sum NB values per lane over a warp (transpose reduction): lane l ends with
-// the warp sum of value (l >> (5 - log2 NB)) & (NB - 1).
-template <int NB>
-BSOFI_DEVINL double wsum_t(double (&v)[NB], int lane) {
-  constexpr int LOG = (NB == 16) ? 4 : 3;
-#pragma unroll
-  for (int lev = 0; lev < LOG; lev++) {
-    const int off = 16 >> lev, half = NB >> (lev + 1);
-    const bool up = (lane & off) != 0;
-#pragma unroll
-    for (int j = 0; j < half; j++) {
-      double send = up ? v[j] : v[j + half];
-      double keep = up ? v[j + half] : v[j];
-      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-  double s = v[0];
-#pragma unroll
-  for (int off = 16 >> LOG; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  return s;
-}
-
-template <int NB>
-struct Smem {
-  double red[2][BW][NB];
-  double coef[2][NB + 4];   // tau*w_c (c < NB), tau, scale, beta
-  double prow[2][NB];
-  double gsh[2][NB];
-  double T[NB][NB + 1];
-  double redW[BW][NB][NB + 1];
-  double W[NB][NB + 1];
+template <int MW>
+struct ChainSmem {
+  // Two buffers, of even and odd columns; columns in the lane groups' order
+  // (g, then 8 + g).
+  double red[2][16 * MW];  // per column: one partial dot product per warp
+  double prow[2][16];      // pivot row
+  double sc[16];           // 1/(alpha - beta) of the finished columns
+  double vtv[2][17];       // v_j^T v_I of the finished columns j < I, and tau_I
+  alignas(16) double top[16 * 16];     // pivot rows of the next leaf on their way to the top warp
+  // T, and (once every warp has used it) W^T T in the same place.
+  union {
+    double T[16][17];
+    alignas(16) double W[256];
+  };
+  ChainStep step[2];       // of leaves s, s+1
+  uint64_t bar;            // bulk loads
   int flag;
   int task;
-  int pflag;  // next-tile prefetch of the panel CTA succeeded
 };
 
-// T(0:I, I) = -tau_I T(0:I,0:I) g_I (LAPACK dlarft), run by one warp one
-// column behind the factorization; T and g are zero outside their ranges.
-template <int NB>
-BSOFI_DEVINL void t_column(Smem<NB>& sm, int I, int lane) {
-  const int buf = I & 1;
-  const double taui = sm.coef[buf][NB];
-  if (lane < I) {
-    double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-    for (int b = 0; b < NB; b += 2) {
-      s0 = fma(sm.T[lane][b], sm.gsh[buf][b], s0);
-      s1 = fma(sm.T[lane][b + 1], sm.gsh[buf][b + 1], s1);
-    }
-    sm.T[lane][I] = -taui * (s0 + s1);
-  }
-  if (lane == I) sm.T[I][I] = taui;
-  __syncwarp();
+// Tiles in shared memory are plain column-major, so that one bulk copy moves
+// a column.  The column stride is 2 mod 16 doubles and the lane group g owns
+// columns col_of(g) and col_of(g) + 8 (not g and g + 8): then both fragment
+// patterns, 16-byte row pairs of two groups' columns and single rows of every
+// second column, touch every bank once.
+BSOFI_DEVINL int col_of(int g) { return (g >> 1) + 4 * (g & 1); }
+BSOFI_DEVINL int group_of(int c) { return 2 * (c & 3) + ((c >> 2) & 1); }  // c = 0..7
+BSOFI_DEVINL int sidx(int r, int c, int S) { return c * S + r; }
+// Column stride of a panel's tile (2n rows, rounded up to 16).
+__host__ __device__ __forceinline__ int tile_stride(int n) { return ((2 * n + 15) & ~15) + 2; }
+
+// Bulk copies of one column between global and shared memory (16-byte
+// aligned, a multiple of 16 bytes), off the load/store pipe that the
+// computing warps need.
+BSOFI_DEVINL void bulk_load(double* dst, const double* src, int rows, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+          tc::smem_u32(dst)),
+      "l"(src), "r"(rows * 8), "r"(tc::smem_u32(bar))
+      : "memory");
+}
+BSOFI_DEVINL void bulk_store(double* dst, const double* src, int rows) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+               "r"(tc::smem_u32(src)), "r"(rows * 8)
+               : "memory");
+}
+BSOFI_DEVINL void bulk_store_wait() {
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+// Between this thread's generic accesses (and those it has synchronised with)
+// and asynchronous copies of the same memory.
+BSOFI_DEVINL void fence_proxy() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
+// Bounded wait for the bulk loads of one phase; reports through the error word.
+BSOFI_DEVINL bool bulk_wait(uint64_t* bar, uint32_t parity, int* err) {
+  for (int i = 0; i < (1 << 22); i++)
+    if (tc::mbar_try_wait(bar, parity)) return true;
+  atomicExch(err, 1);
+  return false;
 }
 
-// Householder QR of one leaf held in registers (thread t owns rows t + BT*i).
-// The column loop is a runtime loop over a rotating layout: at step I
-// position 0 holds column I, positions 1..NB-1-I the columns not yet
-// factored, and positions NB-I..NB-1 the finished reflectors 0..I-1; the
-// array rotates left by one position after each step, so every register index
-// is a compile-time constant while the loop body exists once (a fully
-// unrolled column loop overflows the instruction cache).
-//
-// One block reduction per column carries, per position, either the dot
-// product d_c = sum_{r>I} a_rI a_rc with a pending column (position 0 gives
-// ||x||^2) or e_j = sum_{r>I} v_j[r] a_rI with a finished reflector, which
-// builds the dlarft factor T(0:I,I) = -tau_I T(0:I,0:I) V^T v_I.
-template <int R, int NB, int FW>
-BSOFI_DEVINL void factor_leaf(double (&a)[R][NB], Smem<NB>& sm, int m, int w, double* tau_out) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int SH = (NB == 16) ? 1 : 2;
-  constexpr int FT = FW * 32;  // threads taking part; thread t owns rows t + FT*i
-  auto bar = [&]() {
-    if constexpr (FW == BW) __syncthreads();
-    else named_bar(FT);
+template <int COUNT>
+BSOFI_DEVINL void bar_main() {
+  asm volatile("bar.sync 1, %0;" ::"n"(COUNT) : "memory");
+}
+// Column step barrier: the factoring warps and the T warp.
+template <int COUNT>
+BSOFI_DEVINL void bar_col() {
+  asm volatile("bar.sync 4, %0;" ::"n"(COUNT) : "memory");
+}
+template <int COUNT>
+BSOFI_DEVINL void bar_all() {
+  asm volatile("bar.sync 3, %0;" ::"n"(COUNT) : "memory");
+}
+template <int COUNT>
+BSOFI_DEVINL void bar_help() {
+  asm volatile("bar.sync 2, %0;" ::"n"(COUNT) : "memory");
+}
+
+BSOFI_DEVINL double shfl_d(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+BSOFI_DEVINL double shfl_x(double v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
+
+// One thread's bounded wait until *p >= target; false when it gave up.
+BSOFI_DEVINL bool wait_geq(const BsofState& st, const int* p, int target) {
+  long long it = 0;
+  while (ld_acquire(p) < target) {
+    if (ld_acquire(st.err) != 0) return false;
+    if (++it > st.spin_limit) {
+      atomicExch(st.err, 1);
+      return false;
+    }
+    __nanosleep(32);
+  }
+  return true;
+}
+
+// Rows r, r+1 of one column in global memory (through L2: the tile may have
+// been written by another SM).  vec: the pair is 16-byte aligned.
+BSOFI_DEVINL double2 ld_pair(const double* col, int r, int rows, bool ok, bool vec) {
+  double2 v = make_double2(0.0, 0.0);
+  if (ok) {
+    if (vec && r + 1 < rows) {
+      v = __ldcg(reinterpret_cast<const double2*>(col + r));
+    } else {
+      if (r < rows) v.x = __ldcg(col + r);
+      if (r + 1 < rows) v.y = __ldcg(col + r + 1);
+    }
+  }
+  return v;
+}
+BSOFI_DEVINL void st_pair(double* col, int r, int rows, bool ok, bool vec, double x, double y) {
+  if (!ok) return;
+  if (vec && r + 1 < rows) {
+    __stcg(reinterpret_cast<double2*>(col + r), make_double2(x, y));
+  } else {
+    if (r < rows) __stcg(col + r, x);
+    if (r + 1 < rows) __stcg(col + r + 1, y);
+  }
+}
+BSOFI_DEVINL bool pair_aligned(const double* p, long long ld) {
+  return ((reinterpret_cast<uintptr_t>(p) & 15) == 0) && ((ld & 1) == 0);
+}
+
+// ------------------------------------------------------------ column steps
+struct Refl {
+  double tau, scale, beta, q;  // q = tau * scale = -1 / beta
+};
+// LAPACK dlarfg: beta = -sign(alpha) ||(alpha, x)||, tau = (beta - alpha)/beta
+// = 1 + |alpha|/||.||, scale = 1/(alpha - beta).  The square root, its
+// reciprocal and 1/(|alpha| + ||.||) are the longest dependent chain of a
+// column step, so they share one: Goldschmidt's coupled iteration (Markstein,
+// "Software division and square root using Goldschmidt's algorithms", 2004)
+// from the hardware's approximation gives norm and half its reciprocal
+// together, Newton's residual step finishes each, and the last reciprocal
+// starts from the first norm estimate meanwhile.  Against long double on 10^6
+// random pairs the largest errors are, in units of 2^-53, beta 1.48, tau 1.40, scale
+// 2.62 (with rsqrt() and a division: beta 1.92, scale 3.04).  Outside the range
+// where the approximations are normal numbers those functions are called.
+BSOFI_DEVINL Refl reflector(double xnorm2, double alpha) {
+  Refl r;
+  const double s2 = fma(alpha, alpha, xnorm2), aa = fabs(alpha);
+  // Every lane holds the same values: one vote keeps the branch uniform.
+  const unsigned hi = __double2hiint(s2);  // [2^-930, 2^930) or not
+  const bool rare = xnorm2 == 0.0 || hi - 0x05d00000u >= 0x74400000u;
+  const unsigned any = __any_sync(0xffffffffu, rare);
+  double y, z;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s2));
+  double nrm = s2 * y, h = 0.5 * y;
+  const double est = aa + nrm;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(z) : "d"(est));
+  const double e = fma(-nrm, h, 0.5);
+  nrm = fma(nrm, e, nrm);
+  h = fma(h, e, h);
+  nrm = fma(fma(-nrm, nrm, s2), h, nrm);
+  double rn = h + h;
+  rn = fma(rn, fma(-nrm, rn, 1.0), rn);
+  const double d = fma(-(aa + nrm), z, 1.0);
+  z = fma(z, fma(d, d, d), z);
+  r.beta = -copysign(nrm, alpha);
+  r.tau = fma(aa, rn, 1.0);
+  r.scale = copysign(z, alpha);
+  r.q = copysign(rn, alpha);
+  if (any) {
+    if (xnorm2 == 0.0) {
+      r.tau = 0.0;
+      r.beta = alpha;
+      r.scale = 1.0;
+      r.q = 0.0;
+    } else {
+      const double rs = rsqrt(s2);
+      r.beta = -copysign(s2 * rs, alpha);
+      r.tau = fma(aa, rs, 1.0);
+      r.scale = 1.0 / (alpha - r.beta);
+      r.q = copysign(rs, alpha);
+    }
+  }
+  return r;
+}
+
+// Sum over the four lanes t of a column's group (lane 4 g + t), to all four:
+// one DMMA with a matrix of ones (27 cycles against about 70 for two shuffle
+// and add levels).
+BSOFI_DEVINL double quad_sum(double v) {
+  double d[2] = {0.0, 0.0};
+  dmma_8x8x4(d, v, 1.0);
+  return d[0];
+}
+
+// Sum over the warps' partials of a column (c in the lane groups' order).
+template <int MW>
+BSOFI_DEVINL double col_total(const double* red, int c, int t) {
+  if constexpr (MW == 8) {
+    const double2 a = *reinterpret_cast<const double2*>(red + c * 8 + 2 * t);
+    return quad_sum(a.x + a.y);
+  } else {
+    return quad_sum(red[c * 4 + t]);
+  }
+}
+
+// Warp sums of the two columns' partial dot products into red[column][warp]:
+// again DMMAs with ones, whose results lane 4 g + t holds for columns 2t, 2t+1.
+template <int MW>
+BSOFI_DEVINL void put_partials(double* red, double d0, double d1, int g, int t, int warp) {
+  double e0[2] = {0.0, 0.0}, e1[2] = {0.0, 0.0};
+  dmma_8x8x4(e0, 1.0, d0);
+  dmma_8x8x4(e1, 1.0, d1);
+  if (g < 2) {
+    double* dst = red + (8 * g + 2 * t) * MW + warp;
+    dst[0] = g == 0 ? e0[0] : e1[0];
+    dst[MW] = g == 0 ? e0[1] : e1[1];
+  }
+}
+
+// One pass of a row warp over its rows: the update by the finished pivot
+// column I (half CSU; factors f0, f1 for columns g, g+8, zero where a column
+// is finished; UPD0: some of columns g are pending) and the dot products with
+// the next pivot column J = I+1 (half CSD).  ab8: first 8-row block of the
+// leaf; nb: row blocks of the panel.
+template <class K, bool UPD0, int CSU, int CSD>
+BSOFI_DEVINL void row_pass(double (&a)[K::NI][2][2], double (&x)[K::KEEPX ? K::NI : 1][2],
+                           double f0, double f1, int srcu, int srcd, int ab8, int nb, int warp,
+                           double& d0, double& d1) {
+  double s0[2] = {0.0, 0.0}, s1[2] = {0.0, 0.0};
+#pragma unroll
+  for (int q = 0; q < K::NG; q++) {
+    constexpr int GS = K::GS;
+    const int ia = q * GS, ie = (ia + GS < K::NI ? ia + GS : K::NI);
+    if ((ie - 1) * K::FW + warp < ab8 || 2 + ia * K::FW + warp >= nb) continue;
+#pragma unroll
+    for (int i = ia; i < ie; i++) {
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        double xo;
+        if constexpr (K::KEEPX) xo = x[i][h];
+        else xo = shfl_d(a[i][CSU][h], srcu);
+        if (UPD0) a[i][0][h] = fma(-xo, f0, a[i][0][h]);
+        a[i][1][h] = fma(-xo, f1, a[i][1][h]);
+        const double xn = shfl_d(a[i][CSD][h], srcd);
+        if constexpr (K::KEEPX) x[i][h] = xn;
+        s0[h] = fma(xn, a[i][0][h], s0[h]);
+        s1[h] = fma(xn, a[i][1][h], s1[h]);
+      }
+    }
+  }
+  d0 = s0[0] + s0[1];
+  d1 = s1[0] + s1[1];
+}
+
+// The dot products with column 0, before the first column step.
+template <class K>
+BSOFI_DEVINL void row_first(double (&a)[K::NI][2][2], double (&x)[K::KEEPX ? K::NI : 1][2], int t,
+                            double& d0, double& d1) {
+  double s0[2] = {0.0, 0.0}, s1[2] = {0.0, 0.0};
+#pragma unroll
+  for (int i = 0; i < K::NI; i++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const double xn = shfl_d(a[i][0][h], t);
+      if constexpr (K::KEEPX) x[i][h] = xn;
+      s0[h] = fma(xn, a[i][0][h], s0[h]);
+      s1[h] = fma(xn, a[i][1][h], s1[h]);
+    }
+  d0 = s0[0] + s0[1];
+  d1 = s1[0] + s1[1];
+}
+
+// Sums, reflector and v_I^T a_c of this lane's columns at column step I.
+struct ColStep {
+  Refl rf;
+  double w0, w1;
+};
+template <int MW>
+BSOFI_DEVINL ColStep col_step(const ChainSmem<MW>& sm, int I, int g, int t) {
+  const int buf = I & 1, ri = group_of(I & 7) + (I & 8);
+  ColStep c;
+  const double alpha = sm.prow[buf][ri], pr0 = sm.prow[buf][g], pr1 = sm.prow[buf][g + 8];
+  const double sp = col_total<MW>(sm.red[buf], ri, t);
+  const double s0 = col_total<MW>(sm.red[buf], g, t);
+  const double s1 = col_total<MW>(sm.red[buf], g + 8, t);
+  c.rf = reflector(sp, alpha);
+  // v_I^T a_c = a_Ic + scale d_c.
+  c.w0 = fma(c.rf.scale, s0, pr0);
+  c.w1 = fma(c.rf.scale, s1, pr1);
+  return c;
+}
+
+// The column loop of a row warp.
+template <class K>
+BSOFI_DEVINL void factor_rows(double (&a)[K::NI][2][2], ChainSmem<K::MW>& sm, int w, int ab8,
+                              int nb, int g, int t, int warp) {
+  constexpr int MW = K::MW;
+  const int c0 = col_of(g), c1 = c0 + 8;
+  double x[K::KEEPX ? K::NI : 1][2];
+  double d0, d1;
+  row_first<K>(a, x, t, d0, d1);
+  put_partials<MW>(sm.red[0], d0, d1, g, t, warp);
+  int I = 0;
+  auto step = [&](auto upd0, auto csu, auto csd) {
+    bar_col<K::CT>();
+    const ColStep c = col_step<MW>(sm, I, g, t);
+    const double f0 = c0 > I ? c.rf.q * c.w0 : 0.0, f1 = c1 > I ? c.rf.q * c.w1 : 0.0;
+    const int su = group_of(I & 7) * 4 + t, sd = group_of((I + 1) & 7) * 4 + t;
+    row_pass<K, upd0.value != 0, csu.value, csd.value>(a, x, f0, f1, su, sd, ab8, nb, warp, d0,
+                                                       d1);
+    put_partials<MW>(sm.red[(I + 1) & 1], d0, d1, g, t, warp);
   };
+  using Z = std::integral_constant<int, 0>;
+  using O = std::integral_constant<int, 1>;
+  const int last = w - 1;
 #pragma unroll 1
-  for (int I = 0; I < w; I++) {
-    const int buf = I & 1;
-    const int ndone0 = NB - I;  // first position holding a finished reflector
-    if (tid == I) {
-#pragma unroll
-      for (int p = 0; p < NB; p++) sm.prow[buf][p] = a[0][p];
-    }
-    double part[NB];
-#pragma unroll
-    for (int p = 0; p < NB; p++) part[p] = 0.0;
-#pragma unroll
-    for (int i = 0; i < R; i++) {
-      const int r = tid + FT * i;
-      const double x = (r > I) ? a[i][0] : 0.0;  // rows >= m hold zeros
-#pragma unroll
-      for (int p = 0; p < NB; p++) part[p] = fma(x, a[i][p], part[p]);
-    }
-    {
-      double sum = wsum_t<NB>(part, lane);
-      if ((lane & ((1 << SH) - 1)) == 0) sm.red[buf][warp][(lane >> SH) & (NB - 1)] = sum;
-    }
-    bar();
-    if (warp == 0) {
-      const int slot = lane % NB;
-      double tot = 0.0;
-#pragma unroll
-      for (int k = lane / NB; k < FW; k += 32 / NB) tot += sm.red[buf][k][slot];
-#pragma unroll
-      for (int off = NB; off < 32; off <<= 1) tot += __shfl_xor_sync(0xffffffffu, tot, off);
-      const double xnorm2 = __shfl_sync(0xffffffffu, tot, 0);
-      const double alpha = sm.prow[buf][0];
-      double beta, taui, scale;
-      if (xnorm2 == 0.0) {
-        taui = 0.0;
-        beta = alpha;
-        scale = 1.0;
-      } else {
-        // beta = -sign(alpha) ||(alpha, x)||, tau = (beta - alpha)/beta = 1 + |alpha|/||.||,
-        // scale = 1/(alpha - beta): one reciprocal square root and one division.
-        const double s2 = fma(alpha, alpha, xnorm2);
-        const double rn = rsqrt(s2);
-        beta = -copysign(s2 * rn, alpha);
-        taui = fma(fabs(alpha), rn, 1.0);
-        scale = 1.0 / (alpha - beta);
-      }
-      const double val = fma(scale, tot, sm.prow[buf][slot]);
-      if (lane < NB) {
-        // tau*w_c at pending positions 1..NB-1-I, zero elsewhere, so the row
-        // update below needs no predicates.
-        sm.coef[buf][slot] = (slot >= 1 && slot < ndone0) ? taui * val : 0.0;
-        // g_j = v_j^T v_I for j < I, zero for j >= I.
-        // lane slot writes g at index (slot - ndone0) mod NB: indices < I get
-        // the reflector dot products, the others zero.
-        const int j = (slot + I) & (NB - 1);
-        sm.gsh[buf][j] = (slot >= ndone0) ? val : 0.0;
-      }
-      if (lane == 0) {
-        sm.coef[buf][NB] = taui;
-        sm.coef[buf][NB + 1] = scale;
-        sm.coef[buf][NB + 2] = beta;
-        tau_out[I] = taui;
-      }
-    }
-    if (warp == 1 && I > 0) t_column<NB>(sm, I - 1, lane);
-    bar();
-    const double taui = sm.coef[buf][NB], scale = sm.coef[buf][NB + 1],
-                 beta = sm.coef[buf][NB + 2];
-    double cf[NB];
-#pragma unroll
-    for (int p = 1; p < NB; p++) cf[p] = sm.coef[buf][p];
-#pragma unroll
-    for (int i = 0; i < R; i++) {
-      const int r = tid + FT * i;
-      const double sv = a[i][0] * scale;
-      const double v = (r > I) ? sv : ((r == I) ? 1.0 : 0.0);
-      a[i][0] = (r > I) ? sv : ((r == I) ? beta : a[i][0]);
-#pragma unroll
-      for (int p = 1; p < NB; p++) a[i][p] = fma(-v, cf[p], a[i][p]);
-    }
-    // Rotate left: the finished column moves to the last position.
-#pragma unroll
-    for (int i = 0; i < R; i++) {
-      const double t0 = a[i][0];
-#pragma unroll
-      for (int p = 0; p < NB - 1; p++) a[i][p] = a[i][p + 1];
-      a[i][NB - 1] = t0;
-    }
-  }
-  bar();
-  if (warp == 1) t_column<NB>(sm, w - 1, lane);
-  bar();
-  // A leaf narrower than NB needs NB - w more rotations to restore column order.
+  for (; I < min(last, 7); I++) step(O{}, Z{}, Z{});
+  if (I < last) {  // I = 7
+    step(Z{}, Z{}, O{});
+    I++;
 #pragma unroll 1
-  for (int k = w; k < NB; k++) {
-#pragma unroll
-    for (int i = 0; i < R; i++) {
-      const double t0 = a[i][0];
-#pragma unroll
-      for (int p = 0; p < NB - 1; p++) a[i][p] = a[i][p + 1];
-      a[i][NB - 1] = t0;
-    }
+    for (; I < last; I++) step(Z{}, O{}, O{});
   }
+  bar_col<K::CT>();  // the last column's sums are there
+  bar_col<K::CT>();  // and its scale
 }
 
-// 16-wide block reflector applied with DMMA (mma.sync m16n8k4 f64):
-//   W = V^T C (16 x 16, K = rows split over the 8 warps), W <- -T^T W,
-//   C <- C + V W (rows split over the warps).
-// sV, sC: MP x 20 row-major tiles in shared memory (rows >= m are zero); the
-// caller fills sV, this function stages C.  A stride of 20 doubles makes the
-// fragment loads of both products bank-conflict free.
-constexpr int MS = 20;
-
-// Rows of one staging pass: two thread-owned row slices (R >= 2), i.e. the
-// staged tiles never exceed 2 * BT rows whatever the leaf height.
-template <int R>
-struct Pass {
-  static constexpr int SL = R >= 2 ? 2 : 1;      // row slices per pass
-  static constexpr int ROWS = SL * BT;           // staged rows per pass
-  static constexpr int NP = (R + SL - 1) / SL;   // passes
-  // V is staged column-major with this column stride (ROWS + 4: 4 mod 16
-  // doubles), so that writes of whole rows by their owning threads and both
-  // DMMA fragment patterns read below are free of bank conflicts.
-  static constexpr int SV = ROWS + 4;
-};
-
-// Fill the staged V rows of pass p.  From registers (the factoring CTA) when
-// VREG, else from the stored reflectors in global memory.
-template <int R, bool VREG>
-BSOFI_DEVINL void stage_v(double* sV, const double (&a)[R][16], const double* P, long long ld,
-                          int m, int w, int p) {
-  constexpr int SL = Pass<R>::SL;
-  const int tid = threadIdx.x;
+// The top warp's 16 pivot rows (blocks 0, 1 in a[0], a[1]): update by pivot
+// column I (half CSU; rows below I; row I by v_I = 1, its pivot entry becomes
+// beta).
+template <class K, int CSU>
+BSOFI_DEVINL void top_update(double (&a)[K::NI][2][2], const double (&x)[2][2], const Refl& rf,
+                             double F0, double F1, int I, int g, int t) {
 #pragma unroll
-  for (int j = 0; j < SL; j++) {
-    const int i = p * SL + j;
-    const int lr = tid + BT * j;          // row inside the pass
-    const int r = tid + BT * i;           // row of the leaf
+  for (int b = CSU; b < 2; b++)
 #pragma unroll
-    for (int c = 0; c < 16; c++) {
-      double v = 0.0;
-      if (i < R && r < m && c < w) {
-        if (r == c) v = 1.0;
-        else if (r > c) v = VREG ? a[i < R ? i : 0][c] : __ldcg(P + cm(r, c, ld));
+    for (int h = 0; h < 2; h++) {
+      const int row = 8 * b + 2 * t + h;
+      const double v = row == I ? 1.0 : x[b][h] * rf.scale;
+      if (CSU == 0) a[b][0][h] = fma(-v, F0, a[b][0][h]);
+      a[b][1][h] = fma(-v, F1, a[b][1][h]);
+      if (b == CSU && row == I && g == group_of(I & 7)) a[b][CSU][h] = rf.beta;
+    }
+}
+
+// Dot products with column J (half CSD) over rows below J, and row J to prow.
+template <class K, int CSD>
+BSOFI_DEVINL void top_dots(const double (&a)[K::NI][2][2], double (&x)[2][2], int J, int g, int t,
+                           double* prow, double& d0, double& d1) {
+  const int src = group_of(J & 7) * 4 + t;
+  d0 = d1 = 0.0;
+#pragma unroll
+  for (int b = CSD; b < 2; b++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int row = 8 * b + 2 * t + h;
+      const double xs = shfl_d(a[b][CSD][h], src);
+      x[b][h] = row > J ? xs : 0.0;
+      d0 = fma(x[b][h], a[b][0][h], d0);
+      d1 = fma(x[b][h], a[b][1][h], d1);
+      if (b == CSD && row == J) {
+        prow[g] = a[b][0][h];
+        prow[g + 8] = a[b][1][h];
       }
-      sV[c * Pass<R>::SV + lr] = v;
     }
-  }
 }
 
-// Staged C of pass p: row-major with stride MS.  Each warp instruction copies
-// an 8-row x 4-column block (lane = 4 * row + column), which reads four 64-byte
-// column segments from global memory and writes shared memory without bank
-// conflicts.  Staged row lr is row p * ROWS + lr of the tile.  NW warps take
-// part; wid is this warp's index among them.
-template <int R, int NW = BW>
-BSOFI_DEVINL void stage_c(double* sC, const double* C, long long ld, int m, int w, int p,
-                          int wid = threadIdx.x >> 5) {
-  constexpr int PR = Pass<R>::ROWS, NBK = PR / 8 * 4 / NW;  // blocks per warp
-  constexpr int CH = NBK > 32 ? 32 : NBK;                   // loads in flight per chunk
-  const int lane = threadIdx.x & 31;
-  const int rg = lane >> 2, cg = lane & 3;
-#pragma unroll
-  for (int q0 = 0; q0 < NBK; q0 += CH) {
-    double v[CH];
-#pragma unroll
-    for (int q = 0; q < CH; q++) {
-      const int b = wid + NW * (q0 + q);
-      const int lr = (b >> 2) * 8 + rg, cc = (b & 3) * 4 + cg;
-      const int r = p * PR + lr;
-      v[q] = (r < m && cc < w) ? __ldcg(C + cm(r, cc, ld)) : 0.0;
+// The column loop of the top warp.
+template <class K>
+BSOFI_DEVINL void factor_top(double (&a)[K::NI][2][2], ChainSmem<K::MW>& sm, int w, int g, int t,
+                             double* tau) {
+  constexpr int MW = K::MW;
+  const int c0 = col_of(g), c1 = c0 + 8;
+  double x[2][2], d0, d1, sc0 = 0.0, sc1 = 0.0;
+  top_dots<K, 0>(a, x, 0, g, t, sm.prow[0], d0, d1);
+  put_partials<MW>(sm.red[0], d0, d1, g, t, K::FW);
+  int I = 0;
+  auto step = [&](auto csu, auto csd, auto dot) {
+    bar_col<K::CT>();
+    const ColStep c = col_step<MW>(sm, I, g, t);
+    const double F0 = c0 > I ? c.rf.tau * c.w0 : 0.0, F1 = c1 > I ? c.rf.tau * c.w1 : 0.0;
+    top_update<K, csu.value>(a, x, c.rf, F0, F1, I, g, t);
+    if (dot.value) {
+      top_dots<K, csd.value>(a, x, I + 1, g, t, sm.prow[(I + 1) & 1], d0, d1);
+      put_partials<MW>(sm.red[(I + 1) & 1], d0, d1, g, t, K::FW);
     }
-#pragma unroll
-    for (int q = 0; q < CH; q++) {
-      const int b = wid + NW * (q0 + q);
-      sC[((b >> 2) * 8 + rg) * MS + (b & 3) * 4 + cg] = v[q];
+    // v_j^T v_I of the finished columns j < I (both unscaled in registers,
+    // row I of v_I is 1) for the T warp.
+    if (t == 0) {
+      double* v = sm.vtv[I & 1];
+      v[c0] = c0 < I ? sc0 * c.w0 : 0.0;
+      v[c1] = c1 < I ? sc1 * c.w1 : 0.0;
+      if (g == 0) {
+        v[16] = c.rf.tau;
+        tau[I] = c.rf.tau;
+        sm.sc[I] = c.rf.scale;
+      }
     }
-  }
-}
-
-// 16-wide block reflector applied with DMMA (mma.sync m16n8k8 f64), in passes
-// of at most 2*BT rows staged in shared memory:
-//   W = V^T C (16 x 16; K = rows, split over the 8 warps, summed over passes),
-//   W <- -T^T W,  C <- C + V W  (second sweep over the passes).
-// A stride of MS = 20 doubles makes the fragment loads bank-conflict free.
-// wv: width of the leaf (reflector columns), w: width of the target tile.
-// VPRE / CPRE: the caller already staged V / C (single pass only).
-template <int R, bool VREG, bool VPRE = false, bool CPRE = false>
-BSOFI_DEVINL void apply_qt_mma(double* sV, double* sC, const double (&a)[R][16],
-                               const double* P, long long ldp, int wv, double* C, long long ld,
-                               int m, int w, Smem<16>& sm) {
-  static_assert(!VPRE || Pass<R>::NP == 1, "pre-staged V needs a single pass");
-  static_assert(!CPRE || Pass<R>::NP == 1, "pre-staged C needs a single pass");
-  constexpr int PR = Pass<R>::ROWS, NP = Pass<R>::NP;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+    if (I == c0) sc0 = c.rf.scale;
+    if (I == c1) sc1 = c.rf.scale;
+  };
+  using Z = std::integral_constant<int, 0>;
+  using O = std::integral_constant<int, 1>;
+  const int last = w - 1;
 #pragma unroll 1
-  for (int p = 0; p < NP; p++) {
-    if (!VPRE) stage_v<R, VREG>(sV, a, P, ldp, m, wv, p);
-    if (!CPRE) stage_c<R>(sC, C, ld, m, w, p);
-    __syncthreads();
-    constexpr int KW = PR / BW;
-    const int r0 = warp * KW;
-#pragma unroll 2
-    for (int k0 = r0; k0 < r0 + KW; k0 += 8) {
-      constexpr int SV = Pass<R>::SV;
-      const double a0 = sV[g * SV + k0 + t], a1 = sV[(g + 8) * SV + k0 + t];
-      const double a2 = sV[g * SV + k0 + t + 4], a3 = sV[(g + 8) * SV + k0 + t + 4];
-      dmma_16x8x8(acc[0], a0, a1, a2, a3, sC[(k0 + t) * MS + g], sC[(k0 + t + 4) * MS + g]);
-      dmma_16x8x8(acc[1], a0, a1, a2, a3, sC[(k0 + t) * MS + 8 + g],
-                  sC[(k0 + t + 4) * MS + 8 + g]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int j = 0; j < 2; j++) {
-    sm.redW[warp][g][8 * j + 2 * t] = acc[j][0];
-    sm.redW[warp][g][8 * j + 2 * t + 1] = acc[j][1];
-    sm.redW[warp][g + 8][8 * j + 2 * t] = acc[j][2];
-    sm.redW[warp][g + 8][8 * j + 2 * t + 1] = acc[j][3];
-  }
-  __syncthreads();
-  {
-    const int ai = tid & 15, cc = tid >> 4;
-    double s2 = 0.0;
-#pragma unroll
-    for (int k = 0; k < BW; k++) s2 += sm.redW[k][ai][cc];
-    sm.W[ai][cc] = s2;
-  }
-  __syncthreads();
-  {  // -(T^T W); T is zero below its diagonal
-    const int ai = tid & 15, cc = tid >> 4;
-    double s2 = 0.0;
-#pragma unroll
-    for (int b = 0; b < 16; b++) s2 = fma(sm.T[b][ai], sm.W[b][cc], s2);
-    sm.redW[0][ai][cc] = -s2;
-  }
-  __syncthreads();
+  for (; I < min(last, 7); I++) step(Z{}, Z{}, O{});
+  if (I < last) {  // I = 7
+    step(Z{}, O{}, O{});
+    I++;
 #pragma unroll 1
-  for (int p = 0; p < NP; p++) {
-    if (NP > 1) {  // one pass: sV and sC still hold it
-      stage_v<R, VREG>(sV, a, P, ldp, m, wv, p);
-      stage_c<R>(sC, C, ld, m, w, p);
-      __syncthreads();
-    }
-    constexpr int RW = PR / BW;
-#pragma unroll
-    for (int m0 = warp * RW; m0 < (warp + 1) * RW; m0 += 16) {
-#pragma unroll
-      for (int j = 0; j < 2; j++) {
-        double d[4];
-        d[0] = sC[(m0 + g) * MS + 8 * j + 2 * t];
-        d[1] = sC[(m0 + g) * MS + 8 * j + 2 * t + 1];
-        d[2] = sC[(m0 + g + 8) * MS + 8 * j + 2 * t];
-        d[3] = sC[(m0 + g + 8) * MS + 8 * j + 2 * t + 1];
-        constexpr int SV = Pass<R>::SV;
-#pragma unroll
-        for (int k8 = 0; k8 < 16; k8 += 8)
-          dmma_16x8x8(d, sV[(k8 + t) * SV + m0 + g], sV[(k8 + t) * SV + m0 + g + 8],
-                      sV[(k8 + t + 4) * SV + m0 + g], sV[(k8 + t + 4) * SV + m0 + g + 8],
-                      sm.redW[0][k8 + t][8 * j + g], sm.redW[0][k8 + t + 4][8 * j + g]);
-        const int c0 = 8 * j + 2 * t;
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int lr = m0 + g + 8 * h;            // row inside the pass
-          const int i = p * Pass<R>::SL + lr / BT;  // its thread-owned row slice
-          const int rr = (lr % BT) + BT * i;        // row of the leaf
-          if (i < R && rr < m) {
-            if (c0 < w) __stcg(C + cm(rr, c0, ld), d[2 * h]);
-            if (c0 + 1 < w) __stcg(C + cm(rr, c0 + 1, ld), d[2 * h + 1]);
-          }
-        }
-      }
-    }
-    __syncthreads();
+    for (; I < last; I++) step(O{}, O{}, O{});
   }
+  if (I < 8) step(Z{}, Z{}, Z{});
+  else step(O{}, O{}, Z{});
+  bar_col<K::CT>();
 }
 
-// 8-wide block reflector with DMMA m8n8k4 (f64), all rows in one pass:
-//   W = V^T C (8 x 8; K = the leaf's rows, split over the 8 warps),
-//   W <- -T^T W,  C <- C + V W  (rows split over the warps).
-// V and C are staged column-major with column stride S8 = R*BT + 4 (4 mod 16
-// doubles): the staging writes (one row per thread) and the fragment loads of
-// both products are free of bank conflicts.  VREG: V comes from the factoring
-// CTA's registers (thread t owns rows t + BT*i), else from the stored leaf.
-// wv: width of the leaf, w: width of the target tile.
-template <int R>
-struct Stage8 {
-  static constexpr int S8 = R * BT + 4;
-};
-
-template <int R, bool VREG>
-BSOFI_DEVINL void apply_qt_mma8(double* sV, double* sC, const double (&a)[R][8],
-                                const double* P, long long ldp, int wv, double* C, long long ld,
-                                int m, int w, Smem<8>& sm) {
-  constexpr int S8 = Stage8<R>::S8, KW = R * BT / BW;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 2, t = lane & 3;
+// The T warp: column I of T one barrier behind the factorization (LAPACK
+// dlarft): T(0:I,I) = -tau_I T(0:I,0:I) V(:,0:I)^T v_I.  Lane 4 g + t holds
+// rows g and g+8 of columns t, t+4, t+8, t+12.
+BSOFI_DEVINL void t_column(double (&T)[2][4], const double* vtv, int I, int g, int t) {
+  double r0 = 0.0, r1 = 0.0;
 #pragma unroll
-  for (int i = 0; i < R; i++) {
-    const int r = tid + BT * i;
+  for (int q = 0; q < 4; q++) {
+    const double gb = vtv[t + 4 * q];
+    r0 = fma(T[0][q], gb, r0);
+    r1 = fma(T[1][q], gb, r1);
+  }
+  const double tau = vtv[16];
+  r0 = quad_sum(r0);
+  r1 = quad_sum(r1);
+  const double v0 = g == I ? tau : (g < I ? -tau * r0 : 0.0);
+  const double v1 = g + 8 == I ? tau : (g + 8 < I ? -tau * r1 : 0.0);
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-      double v = 0.0;
-      if (r < m && c < wv) {
-        if (r == c) v = 1.0;
-        else if (r > c) v = VREG ? a[i][c] : __ldcg(P + cm(r, c, ldp));
-      }
-      sV[c * S8 + r] = v;
-      sC[c * S8 + r] = (r < m && c < w) ? __ldcg(C + cm(r, c, ld)) : 0.0;
+  for (int q = 0; q < 4; q++)
+    if (I == t + 4 * q) {
+      T[0][q] = v0;
+      T[1][q] = v1;
     }
-  }
-  __syncthreads();
-  {
-    // Four independent accumulators over interleaved 4-deep K steps, so the
-    // DMMAs of a warp do not wait on each other's results.
-    static_assert(KW % 16 == 0, "8-wide W split");
-    double acc[4][2] = {};
-    const int k1 = warp * KW;
-#pragma unroll
-    for (int k0 = k1; k0 < k1 + KW; k0 += 16)
-#pragma unroll
-      for (int q = 0; q < 4; q++)
-        dmma_8x8x4(acc[q], sV[g * S8 + k0 + 4 * q + t], sC[g * S8 + k0 + 4 * q + t]);
-    sm.redW[warp][g][2 * t] = (acc[0][0] + acc[1][0]) + (acc[2][0] + acc[3][0]);
-    sm.redW[warp][g][2 * t + 1] = (acc[0][1] + acc[1][1]) + (acc[2][1] + acc[3][1]);
-  }
-  __syncthreads();
-  if (tid < 64) {
-    const int ai = tid & 7, cc = tid >> 3;
-    double s2 = 0.0;
-#pragma unroll
-    for (int k = 0; k < BW; k++) s2 += sm.redW[k][ai][cc];
-    sm.W[ai][cc] = s2;
-  }
-  __syncthreads();
-  if (tid < 64) {  // -(T^T W); T is zero below its diagonal
-    const int ai = tid & 7, cc = tid >> 3;
-    double s2 = 0.0;
-#pragma unroll
-    for (int b = 0; b < 8; b++) s2 = fma(sm.T[b][ai], sm.W[b][cc], s2);
-    sm.redW[0][ai][cc] = -s2;
-  }
-  __syncthreads();
-#pragma unroll 4
-  for (int m0 = warp * KW; m0 < (warp + 1) * KW; m0 += 8) {
-    double d[2] = {sC[(2 * t) * S8 + m0 + g], sC[(2 * t + 1) * S8 + m0 + g]};
-#pragma unroll
-    for (int k0 = 0; k0 < 8; k0 += 4)
-      dmma_8x8x4(d, sV[(k0 + t) * S8 + m0 + g], sm.redW[0][k0 + t][g]);
-    const int rr = m0 + g;
-    if (rr < m) {
-      if (2 * t < w) __stcg(C + cm(rr, 2 * t, ld), d[0]);
-      if (2 * t + 1 < w) __stcg(C + cm(rr, 2 * t + 1, ld), d[1]);
-    }
-  }
-  __syncthreads();
 }
 
-// FW4: 16-wide leaves of at most 2 BT rows are factored by 4 warps while the
-// other 4 stage the next leaf's tile (true), or by all 8 warps with the tile
-// staged after the factorization (false).
-template <int R, int NB, bool FW4 = true>
-__global__ void __launch_bounds__(BT, 1) bsof_persistent_kernel(BsofGeom g, BsofState st) {
-  __shared__ Smem<NB> sm;
-  extern __shared__ __align__(16) double sC[];  // NB x (R*BT) staged tile
-  const int tid = threadIdx.x;
-  const long long first_task = tasks_before(g, st.s_begin);
-  const long long total_tasks = tasks_before(g, st.s_end);
+// ------------------------------------------------------------ block update
+// Element (c, j) of a 16 x 16 matrix kept row by row with the halves exchanged
+// in rows c = 4..7, 12..15: row pairs (c, c+4) of a quarter-warp access meet
+// different banks.
+BSOFI_DEVINL int widx(int c, int j) { return c * 16 + (j ^ ((c & 4) << 1)); }
 
-  if (blockIdx.x == 0) {
-    // ---------------------------------------------------------- panel chain
-    // 16-wide leaves of at most 2*BT rows are factored by 4 warps with 2R rows
-    // per thread (the per-column shuffle reduction costs per warp); the other
-    // 4 warps meanwhile wait for the next leaf's tile to be ready and stage it
-    // in shared memory for the update that follows (PREFETCH).  Taller leaves
-    // use all warps for the factorization.
-    constexpr int FW = (FW4 && NB == 16 && R <= 2) ? 4 : BW;
-    constexpr int FR = R * BW / FW;
-    constexpr bool PREFETCH = NB == 16 && FW < BW && Pass<R>::NP == 1;
-    const int warp = tid >> 5;
-    // own: this CTA applied the last update to the current leaf's tile, so it
-    // needs no wait (shared barriers order its own global writes).  A launch
-    // that continues at s_begin > 0 starts owning its first tile: the earlier
-    // launch, complete before this one starts, applied that tile's last
-    // update from its panel CTA, which is never counted.
-    bool own = st.s_begin > 0;
+// From this warp's W^T = C^T V over its own rows to the A fragments of
+// -(W^T T) summed over all MW warps.  acc[jt] holds rows c = col_of(g),
+// col_of(g) + 8 and (its B operand having V's columns in the lane groups'
+// order) columns 8 jt + t, 8 jt + t + 4.  The fragments' K index t stands for
+// j = 8 kk + 2t and t + 4 for 8 kk + 2t + 1.  Two barriers among the MW warps.
+template <int MW>
+BSOFI_DEVINL void reduce_w(double (&acc)[2][4], double (&fr)[2][4], double* part, ChainSmem<MW>& sm,
+                           int g, int t, int warp) {
+  // (W^T T): T is upper triangular, so columns 0..7 need only rows 0..7.
+  double o[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+  dmma_16x8x8(o[0], acc[0][0], acc[0][2], acc[0][1], acc[0][3], sm.T[t][g], sm.T[t + 4][g]);
+  dmma_16x8x8(o[1], acc[0][0], acc[0][2], acc[0][1], acc[0][3], sm.T[t][g + 8],
+              sm.T[t + 4][g + 8]);
+  dmma_16x8x8(o[1], acc[1][0], acc[1][2], acc[1][1], acc[1][3], sm.T[8 + t][g + 8],
+              sm.T[12 + t][g + 8]);
+  double* mine = part + warp * 256;
+  const int c0 = col_of(g);
+#pragma unroll
+  for (int jt = 0; jt < 2; jt++)
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+      *reinterpret_cast<double2*>(mine + widx(c0 + 8 * h, 8 * jt + 2 * t)) =
+          make_double2(o[jt][2 * h], o[jt][2 * h + 1]);
+  bar_main<32 * MW>();
+#pragma unroll
+  for (int e = threadIdx.x; e < 256; e += 32 * MW) {
+    double s[MW];
+#pragma unroll
+    for (int k = 0; k < MW; k++) s[k] = part[k * 256 + e];
+#pragma unroll
+    for (int m = MW / 2; m > 0; m /= 2)
+#pragma unroll
+      for (int k = 0; k < m; k++) s[k] += s[k + m];
+    sm.W[e] = -s[0];
+  }
+  bar_main<32 * MW>();
+#pragma unroll
+  for (int kk = 0; kk < 2; kk++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const double2 v =
+          *reinterpret_cast<const double2*>(sm.W + widx(c0 + 8 * h, 8 * kk + 2 * t));
+      fr[kk][h] = v.x;
+      fr[kk][2 + h] = v.y;
+    }
+}
+
+// C^T += fr V^T for the 8-row block at row r0 of V in shared memory.
+BSOFI_DEVINL void update_block(double (&c)[2][2], const double (&fr)[2][4], const double* sV, int SV,
+                               int r0, int g, int t) {
+  double d[4] = {c[0][0], c[0][1], c[1][0], c[1][1]};
+#pragma unroll
+  for (int kk = 0; kk < 2; kk++)
+    dmma_16x8x8(d, fr[kk][0], fr[kk][1], fr[kk][2], fr[kk][3],
+                sV[sidx(r0 + g, 8 * kk + 2 * t, SV)], sV[sidx(r0 + g, 8 * kk + 2 * t + 1, SV)]);
+  c[0][0] = d[0];
+  c[0][1] = d[1];
+  c[1][0] = d[2];
+  c[1][1] = d[3];
+}
+
+// ------------------------------------------------------------ the chain CTA
+// The helper warps: wait for the next tile and (PREF) stage it while the leaf
+// is being factored, build T; store and publish the leaf while the next tile
+// is being updated.
+template <class K>
+BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const double* sV, double* sC,
+                               int SV, ChainSmem<K::MW>& sm) {
+  const int ht = threadIdx.x - K::MT, lane = threadIdx.x & 31, hw = ht >> 5;
+  const int n = g.n, SC = SV + 16, capc = SC - 2;
+  uint32_t phase = 0;
+  constexpr int LW = K::HW - 1;  // loading warps; the last one builds T
+  if (hw == LW) {
+    const int gq = lane >> 2, t = lane & 3;
     for (int s = st.s_begin; s < st.s_end; s++) {
-      const Leaf f = leaf_of(g, s);
-      int lo, hi;
-      tile_range(g, f.m, f.t, lo, hi);
-      if (tid == 0) st.timeline[4 * s + 0] = gtimer();
-      if (!own && !block_wait_geq(st, st.cnt + tile_id(g, f.m, f.t), hi - lo, &sm.flag)) return;
-      if (tid == 0) st.timeline[4 * s + 1] = gtimer();
-      const int mrows = 2 * g.n - f.j0;
-      long long ldp;
-      double* P = mat_ptr(g, st, (long long)f.k * g.n + f.j0, f.m, f.t * g.NB, ldp);
-      // Target 0 of leaf s: the tile of leaf s+1.
-      const bool next = ntargets(g, f) > 0;
-      int m2 = 0, t2 = 0, lo2 = 0, hi2 = 0;
-      if (next) {
-        target_of(g, f, 0, m2, t2);
-        tile_range(g, m2, t2, lo2, hi2);
+      const Leaf f = sm.step[s & 1].f;
+      double T[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+      for (int I = 0; I <= f.w; I++) {
+        bar_col<K::CT>();
+        if (I > 0) t_column(T, sm.vtv[(I - 1) & 1], I - 1, gq, t);
       }
-      const int x2 = tile_id(g, m2, t2);
-      long long ldc = st.ld;
-      double* C = next ? tile_ptr(g, st, f.k, f.j0, m2, t2, ldc) : nullptr;
-      const int w2 = min(g.NB, g.n - t2 * g.NB);
-      for (int e = tid; e < NB * (NB + 1); e += BT) (&sm.T[0][0])[e] = 0.0;
-      if (tid < 2 * NB) (&sm.gsh[0][0])[tid] = 0.0;
-      if (tid == 0) sm.pflag = 1;
-      __syncthreads();
-      double a[FR][NB];
-      if (tid < FW * 32) {
-#pragma unroll
-        for (int i = 0; i < FR; i++) {
-          const int r = tid + FW * 32 * i;
-#pragma unroll
-          for (int c = 0; c < NB; c++)
-            a[i][c] = (r < mrows && c < f.w) ? __ldcg(P + cm(r, c, ldp)) : 0.0;
-        }
-        factor_leaf<FR, NB, FW>(a, sm, mrows, f.w, st.tau + (long long)f.k * g.n + f.j0);
-#pragma unroll
-        for (int i = 0; i < FR; i++) {
-          const int r = tid + FW * 32 * i;
-          if (r < mrows) {
-#pragma unroll
-            for (int c = 0; c < NB; c++)
-              if (c < f.w) __stcg(P + cm(r, c, ldp), a[i][c]);
-          }
-          if constexpr (NB == 16 && Pass<R>::NP == 1) {  // reflectors for the next-tile update
-            if (r < Pass<R>::ROWS) {
-#pragma unroll
-              for (int c = 0; c < 16; c++)
-                sC[c * Pass<R>::SV + r] = (r >= mrows || c >= f.w) ? 0.0
-                                 : (r == c ? 1.0 : (r > c ? a[i][c] : 0.0));
-            }
-          }
-        }
-      } else {
-        if constexpr (PREFETCH) {
-          if (next) {
-            // Wait (bounded) until every update of the next tile before leaf
-            // s is done, then stage it.
-            constexpr int PT = BT - FW * 32;
-            if (tid == FW * 32) {
-              const int* flag = st.cnt + x2;
-              int ok = 1;
-              long long it = 0;
-              while (ld_acquire(flag) < s - lo2) {
-                if (ld_acquire(st.err) != 0 || ++it > st.spin_limit) {
-                  atomicExch(st.err, 1);
-                  ok = 0;
-                  break;
-                }
-                __nanosleep(64);
-              }
-              sm.pflag = ok;
-            }
-            named_bar2(PT);
-            if (sm.pflag)
-              stage_c<R, BW - FW>(sC + Pass<R>::ROWS * MS, C, ldc, mrows, w2, 0, warp - FW);
-          }
-        }
-      }
-      __syncthreads();
-      if (!sm.pflag) return;
       double* Tout = st.T + ((long long)f.k * st.maxleaves + f.l) * 256;
-      for (int e = tid; e < 256; e += BT) {
-        const int rr = e % 16, cc = e / 16;
-        Tout[e] = (rr < NB && cc < NB && rr < f.w && cc < f.w) ? sm.T[rr][cc] : 0.0;
-      }
-      __syncthreads();
-      // Apply leaf s to the tile of leaf s+1.  That is the tile's last update
-      // and only this CTA reads the tile next, so it is not published; the
-      // leaf itself (reflectors and T) is published after the update, with one
-      // fence for both.
-      if (next) {
-        if (!PREFETCH && !block_wait_geq(st, st.cnt + x2, s - lo2, &sm.flag)) return;
-        if (tid == 0) st.timeline[4 * s + 3] = gtimer();
-        if constexpr (NB == 16) {
-          // V is staged from the factor's registers when one pass covers the
-          // leaf, else re-read from L2 (just written by this CTA).
-          double none[R][16];
-          apply_qt_mma<R, false, Pass<R>::NP == 1, PREFETCH>(
-              sC, sC + Pass<R>::ROWS * MS, none, P, ldp, f.w, C, ldc, mrows, w2, sm);
-        } else {
-          apply_qt_mma8<R, true>(sC, sC + 8 * Stage8<R>::S8, a, P, ldp, f.w, C, ldc, mrows, w2,
-                                 sm);
+#pragma unroll
+      for (int r = 0; r < 2; r++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const int i = gq + 8 * r, j = t + 4 * q;
+          sm.T[i][j] = T[r][q];
+          Tout[i + 16 * j] = T[r][q];
         }
-      }
-      if (tid == 0) {
-        __threadfence();
-        red_release_add(st.factored + s, 1);
-        st.timeline[4 * s + 2] = gtimer();
-      }
-      own = next;
+      bar_all<K::THREADS>();
+      if (!sm.flag) return;
+      if (lane == 0 && s + 1 < st.s_end) sm.step[(s + 1) & 1] = chain_step(g, st, s + 1);
+      if (!K::PREF && sm.step[s & 1].trans) bar_all<K::THREADS>();
+      bar_all<K::THREADS>();
     }
     return;
   }
+  for (int s = st.s_begin; s < st.s_end; s++) {
+    const ChainStep& z = sm.step[s & 1];
+    if (ht == 0)
+      sm.flag = !z.next || wait_geq(st, st.cnt + tile_id(g, z.m2, z.t2), s - z.lo2) ? 1 : 0;
+    if constexpr (K::PREF) {
+      bar_help<32 * LW>();
+      if (z.next && sm.flag) {
+        // Rows [ab, rows) of the tile, then (fresh) the n rows below the panel
+        // at shared rows 8 nb, 8 nb + 1, .. (mod capc; the tile's own rows
+        // above ab leave room).
+        const bool vec = pair_aligned(z.C, z.ldc) && (n & 1) == 0;
+        const int f0 = 8 * z.nb, q0 = min(n, capc - f0);
+        if (vec && K::BULK) {
+          if (ht == 0) {
+            fence_proxy();
+            tc::mbar_arrive_expect_tx(&sm.bar, 8 * z.w2 * (z.rows - z.ab + (z.fresh ? n : 0)));
+            for (int c = 0; c < z.w2; c++) {
+              const double* col = z.C + cm(0, c, z.ldc);
+              bulk_load(sC + sidx(z.ab, c, SC), col + z.ab, z.rows - z.ab, &sm.bar);
+              if (z.fresh) {
+                bulk_load(sC + sidx(f0, c, SC), col + 2 * n, q0, &sm.bar);
+                if (n > q0) bulk_load(sC + sidx(0, c, SC), col + 2 * n + q0, n - q0, &sm.bar);
+              }
+            }
+          }
+        }
+#pragma unroll 1
+        for (int c = hw; c < 16; c += LW) {
+          const double* col = z.C + cm(0, c, z.ldc);
+          if (c >= z.w2) {
+            for (int r = z.ab + lane; r < 8 * z.nb; r += 32) sC[sidx(r, c, SC)] = 0.0;
+            continue;
+          }
+          if (vec && !K::BULK) {
+#pragma unroll 1
+            for (int r = z.ab + 2 * lane; r < z.rows; r += 64)
+              cp_async16(sC + sidx(r, c, SC), col + r, 16);
+            if (z.fresh) {
+#pragma unroll 1
+              for (int q = 2 * lane; q < n; q += 64)
+                cp_async16(sC + sidx(q < q0 ? f0 + q : q - q0, c, SC), col + 2 * n + q, 16);
+            }
+          } else if (!vec) {
+#pragma unroll 4
+            for (int r = z.ab + lane; r < z.rows; r += 32) sC[sidx(r, c, SC)] = __ldcg(col + r);
+            if (z.fresh) {
+#pragma unroll 4
+              for (int q = lane; q < n; q += 32)
+                sC[sidx(q < q0 ? f0 + q : q - q0, c, SC)] = __ldcg(col + 2 * n + q);
+            }
+          }
+          // Zero rows up to a full block.
+          if (z.rows + lane < 8 * z.nb)
+            sC[sidx(z.rows + lane, c, SC)] = 0.0;
+        }
+        if (!K::BULK) {
+          cp_async_commit();
+          cp_async_wait<0>();
+        } else if (vec && ht == 0) {
+          if (!bulk_wait(&sm.bar, phase, st.err)) sm.flag = 0;
+          phase ^= 1;
+        }
+      }
+    }
+    bar_all<K::THREADS>();
+    if (!sm.flag) return;
+    // The reflectors below the pivot rows to global memory.
+    if (ht == 0) st.timeline[4 * s + 3] = gtimer();
+    if constexpr (K::BULK) {
+      const bool vec = pair_aligned(z.P, z.ldp);
+      const int r0 = z.ab + 16;
+      if (vec && ((z.rows - r0) & 1) == 0) {
+        if (ht == 0 && z.rows > r0) {
+          for (int c = 0; c < z.f.w; c++)
+            bulk_store(z.P + cm(r0, c, z.ldp), sV + sidx(r0, c, SV), z.rows - r0);
+          bulk_store_wait();
+          fence_proxy();
+        }
+      } else {
+#pragma unroll 1
+        for (int c = hw; c < z.f.w; c += LW) {
+          double* col = z.P + cm(0, c, z.ldp);
+#pragma unroll 4
+          for (int r = r0 + lane; r < z.rows; r += 32) __stcg(col + r, sV[sidx(r, c, SV)]);
+        }
+      }
+    }
+    if constexpr (K::BULK) bar_help<32 * LW>();
+    if (ht == 0) {
+      __threadfence();
+      red_release_add(st.factored + s, 1);
+    }
+    if (!K::PREF && z.trans) bar_all<K::THREADS>();  // V may be overwritten
+    bar_all<K::THREADS>();
+  }
+}
 
-  // ------------------------------------------------------------ workers
+template <class K>
+BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV, double* part,
+                             double* sC, int SV, ChainSmem<K::MW>& sm) {
+  constexpr int FW = K::FW, NI = K::NI, MW = K::MW, MT = K::MT;
+  // (The shuffle tells the compiler that the warp index is uniform.)
+  const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+  const int gq = lane >> 2, t = lane & 3, gc = col_of(gq);
+  const bool top = warp == FW;
+  const int n = g.n, SC = SV + 16, capc = SC - 2;
+  // Slot i of this warp is 8-row block bb + i bs of the panel.
+  double a[NI][2][2];
+#pragma unroll
+  for (int i = 0; i < NI; i++) a[i][0][0] = a[i][0][1] = a[i][1][0] = a[i][1][1] = 0.0;
+  {
+    const Leaf f = leaf_of(g, st.s_begin);
+    const int base = leaf_base(g, f), ab8 = (f.j0 - base) / 8, rows = 2 * n - base;
+    long long ld;
+    const double* P = mat_ptr(g, st, (long long)f.k * n + base, f.m, f.t * 16, ld);
+    const bool vec = pair_aligned(P, ld);
+#pragma unroll
+    for (int i = 0; i < NI; i++) {
+      const int b = top ? ab8 + i : 2 + i * FW + warp;
+      if (top ? i >= 2 : b < ab8 + 2) continue;
+#pragma unroll
+      for (int cs = 0; cs < 2; cs++) {
+        const int c = gc + 8 * cs;
+        const double2 v = ld_pair(P + cm(0, c, ld), 8 * b + 2 * t, rows, c < f.w, vec);
+        a[i][cs][0] = v.x;
+        a[i][cs][1] = v.y;
+      }
+    }
+  }
+  for (int s = st.s_begin; s < st.s_end; s++) {
+    const ChainStep& z = sm.step[s & 1];  // (written before this loop, then by the T warp)
+    const int w = z.f.w, ab = z.ab, ab8 = ab / 8, rows = z.rows, nb = z.nb, w2 = z.w2;
+    const bool next = z.next, fresh = z.fresh, trans = z.trans;
+    double* C = z.C;
+    const long long ldc = z.ldc;
+    const int blo = top ? ab8 : ab8 + 2, bhi = top ? min(nb, ab8 + 2) : nb;
+    const int bb = top ? ab8 : 2 + warp, bs = top ? 1 : FW;
+    {
+      // ---- factor the leaf
+      if (top) {
+        if (lane == 0) {
+          st.timeline[4 * s + 0] = gtimer();
+          st.timeline[4 * s + 1] = st.timeline[4 * s + 0];
+        }
+        factor_top<K>(a, sm, w, gq, t, st.tau + (long long)z.f.k * n + z.f.j0);
+      } else {
+        factor_rows<K>(a, sm, w, ab8, nb, gq, t, warp);
+      }
+      // ---- V to shared memory, the pivot rows (R and V) to global memory
+      // (columns beyond the leaf's width are zero whatever their scale).
+      const double sc0 = gc < w ? sm.sc[gc] : 0.0, sc1 = gc + 8 < w ? sm.sc[gc + 8] : 0.0;
+      const bool vecp = pair_aligned(z.P, z.ldp);
+      if (top) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+#pragma unroll
+          for (int cs = 0; cs < 2; cs++) {
+            const int c = gc + 8 * cs, r = ab + 8 * i + 2 * t;
+            double o[2], v[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              const double e = a[i][cs][h];
+              const int d = 8 * i + 2 * t + h - c;  // row minus column of the leaf
+              o[h] = d > 0 ? e * (cs == 0 ? sc0 : sc1) : e;
+              v[h] = d > 0 ? o[h] : ((d == 0 && c < w) ? 1.0 : 0.0);
+              a[i][cs][h] = v[h];
+            }
+            st_pair(z.P + cm(0, c, z.ldp), r, rows, c < w, vecp, o[0], o[1]);
+            if (ab8 + i < nb)
+              *reinterpret_cast<double2*>(sV + sidx(r, c, SV)) = make_double2(v[0], v[1]);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < NI; i++) {
+          const int b = bb + i * bs;
+          if (b < blo || b >= bhi) continue;
+#pragma unroll
+          for (int cs = 0; cs < 2; cs++) {
+            const int c = gc + 8 * cs, r = 8 * b + 2 * t;
+#pragma unroll
+            for (int h = 0; h < 2; h++) a[i][cs][h] *= cs == 0 ? sc0 : sc1;
+            if constexpr (!K::BULK)
+              st_pair(z.P + cm(0, c, z.ldp), r, rows, c < w, vecp, a[i][cs][0], a[i][cs][1]);
+            *reinterpret_cast<double2*>(sV + sidx(r, c, SV)) =
+                make_double2(a[i][cs][0], a[i][cs][1]);
+          }
+        }
+      }
+      if constexpr (K::BULK) tc::fence_proxy_async_smem();  // V is stored to global memory by bulk copies
+    }
+    bar_all<K::THREADS>();
+    if (!sm.flag) return;
+    if (next) {
+      // ---- leaf s on the tile of leaf s+1.  That is the tile's last update
+      // and only this CTA reads the tile next, so it stays in registers; its
+      // rows above the next leaf are final and go to global memory.
+      double c[NI][2][2];
+      double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+      const bool vec = pair_aligned(C, ldc);
+      constexpr int GS = K::GS;
+#pragma unroll
+      for (int q = 0; q < K::NG; q++) {
+        const int ia = q * GS, ie = (ia + GS < NI ? ia + GS : NI);
+        const bool any = bb + (ie - 1) * bs >= blo && bb + ia * bs < bhi;
+#pragma unroll
+        for (int i = ia; i < ie; i++) c[i][0][0] = c[i][0][1] = c[i][1][0] = c[i][1][1] = 0.0;
+        if (!any) continue;
+#pragma unroll
+        for (int i = ia; i < ie; i++) {
+          const int b = bb + i * bs, r = 8 * b + 2 * t;
+          const bool live = b >= blo && b < bhi;
+#pragma unroll
+          for (int cs = 0; cs < 2; cs++) {
+            const int cc = gc + 8 * cs;
+            double2 v = make_double2(0.0, 0.0);
+            if constexpr (K::PREF) {
+              if (live) v = *reinterpret_cast<const double2*>(sC + sidx(r, cc, SC));
+            } else {
+              v = ld_pair(C + cm(0, cc, ldc), r, rows, live && cc < w2, vec);
+            }
+            c[i][cs][0] = v.x;
+            c[i][cs][1] = v.y;
+          }
+        }
+        if constexpr (K::VREG) {
+#pragma unroll
+          for (int i = ia; i < ie; i++)
+#pragma unroll
+            for (int jt = 0; jt < 2; jt++)
+              dmma_16x8x8(acc[jt], c[i][0][0], c[i][1][0], c[i][0][1], c[i][1][1], a[i][jt][0],
+                          a[i][jt][1]);
+        }
+      }
+      if constexpr (!K::VREG) {
+#pragma unroll
+        for (int i = 0; i < NI; i++) {
+          const int b = bb + i * bs, r = 8 * b + 2 * t;
+          if (b < blo || b >= bhi) continue;
+#pragma unroll
+          for (int jt = 0; jt < 2; jt++) {
+            const double2 v = *reinterpret_cast<const double2*>(sV + sidx(r, gc + 8 * jt, SV));
+            dmma_16x8x8(acc[jt], c[i][0][0], c[i][1][0], c[i][0][1], c[i][1][1], v.x, v.y);
+          }
+        }
+      }
+      double fr[2][4];
+      reduce_w<MW>(acc, fr, part, sm, gq, t, warp);
+      const bool keep_all = s + 1 == st.s_end;
+#pragma unroll
+      for (int q = 0; q < K::NG; q++) {
+        const int ia = q * GS, ie = (ia + GS < NI ? ia + GS : NI);
+        if (bb + (ie - 1) * bs < blo || bb + ia * bs >= bhi) continue;
+        // (Slots of the group that are not live compute values nobody uses.)
+#pragma unroll
+        for (int i = ia; i < ie; i++)
+          update_block(c[i], fr, sV, SV, 8 * min(bb + i * bs, nb - 1), gq, t);
+      }
+      if (top || keep_all) {
+#pragma unroll
+        for (int i = 0; i < NI; i++) {
+          const int b = bb + i * bs, r = 8 * b + 2 * t;
+          if (b < blo || b >= bhi) continue;
+#pragma unroll
+          for (int cs = 0; cs < 2; cs++)
+            st_pair(C + cm(0, gc + 8 * cs, ldc), r, rows, gc + 8 * cs < w2, vec, c[i][cs][0],
+                    c[i][cs][1]);
+        }
+      }
+      if (!trans) {
+        // Blocks ab8 + 2 and ab8 + 3 become the next leaf's pivot rows.
+#pragma unroll
+        for (int i = 0; i < NI; i++) {
+          const int d = bb + i * bs - (ab8 + 2);
+          const bool live = !top && d >= 0 && bb + i * bs < bhi;
+#pragma unroll
+          for (int cs = 0; cs < 2; cs++) {
+            if (live && d < 2)
+              *reinterpret_cast<double2*>(sm.top + (gc + 8 * cs) * 16 + 8 * d + 2 * t) =
+                  make_double2(c[i][cs][0], c[i][cs][1]);
+#pragma unroll
+            for (int h = 0; h < 2; h++) a[i][cs][h] = live && d >= 2 ? c[i][cs][h] : 0.0;
+          }
+        }
+      } else {
+        // Through shared memory: over the tile just read (PREF), else over V
+        // once the helpers have stored it.
+        double* sX = K::PREF ? sC : sV;
+        const int SX = K::PREF ? SC : SV;
+        if constexpr (!K::PREF) bar_all<K::THREADS>();
+#pragma unroll
+        for (int i = 0; i < NI; i++) {
+          const int b = bb + i * bs;
+          if (b < blo || b >= bhi) continue;
+#pragma unroll
+          for (int cs = 0; cs < 2; cs++)
+            *reinterpret_cast<double2*>(sX + sidx(8 * b + 2 * t, gc + 8 * cs, SX)) =
+                make_double2(c[i][cs][0], c[i][cs][1]);
+        }
+        bar_main<MT>();
+        const int rows2 = fresh ? 2 * n : n;
+#pragma unroll
+        for (int i = 0; i < NI; i++) {
+          const int b = top ? i : 2 + i * FW + warp;
+#pragma unroll
+          for (int cs = 0; cs < 2; cs++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              const int r = 8 * b + 2 * t + h, cc = gc + 8 * cs;
+              double v = 0.0;
+              if ((!top || i < 2) && r < rows2 && cc < w2) {
+                if (r < n) {
+                  v = sX[sidx(n + r, cc, SX)];
+                } else if constexpr (K::PREF) {
+                  int rr = 8 * nb + r - n;
+                  if (rr >= capc) rr -= capc;
+                  v = sC[sidx(rr, cc, SC)];
+                } else {
+                  v = __ldcg(C + cm(n + r, cc, ldc));
+                }
+              }
+              a[i][cs][h] = v;
+            }
+        }
+      }
+    }
+    bar_all<K::THREADS>();
+    if (top) {
+      if (next && !trans) {
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+          for (int cs = 0; cs < 2; cs++) {
+            double2 v = make_double2(0.0, 0.0);
+            if (ab8 + 2 + i < nb)
+              v = *reinterpret_cast<const double2*>(sm.top + (gc + 8 * cs) * 16 + 8 * i + 2 * t);
+            a[i][cs][0] = v.x;
+            a[i][cs][1] = v.y;
+          }
+      }
+      if (lane == 0) st.timeline[4 * s + 2] = gtimer();
+    }
+  }
+}
+
+// ------------------------------------------------------------ workers
+template <class K>
+BSOFI_DEVINL void worker(const BsofGeom& g, const BsofState& st, double* sV, double* part, int SV,
+                         ChainSmem<K::MW>& sm) {
+  constexpr int MW = K::MW, MT = K::MT, NIW = K::NIW;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gq = lane >> 2, t = lane & 3, gc = col_of(gq);
+  uint32_t phase = 0;
+  const long long first_task = tasks_before(g, st.s_begin);
+  const long long total_tasks = tasks_before(g, st.s_end);
   for (;;) {
-    if (tid == 0) sm.task = first_task + atomicAdd(st.next_task, 1);
-    __syncthreads();
-    const long long task = sm.task;
-    __syncthreads();
+    if (tid == 0) sm.task = atomicAdd(st.next_task, 1);
+    bar_main<MT>();
+    const long long task = first_task + sm.task;
     if (task >= total_tasks) return;
     // Leaf of this task: largest s with tasks_before(s) <= task.
     int lo_s = 0, hi_s = g.S - 1;
@@ -838,30 +1047,106 @@ __global__ void __launch_bounds__(BT, 1) bsof_persistent_kernel(BsofGeom g, Bsof
     const int s = lo_s;
     const int q = 1 + (int)(task - tasks_before(g, s));
     const Leaf f = leaf_of(g, s);
-    int m2, t2;
+    int m2, t2, lo2, hi2;
     target_of(g, f, q, m2, t2);
-    int lo2, hi2;
     tile_range(g, m2, t2, lo2, hi2);
     const int x2 = tile_id(g, m2, t2);
-    if (!block_wait_geq(st, st.factored + s, 1, &sm.flag)) return;
-    const int mrows = 2 * g.n - f.j0;
-    const double* T = st.T + ((long long)f.k * st.maxleaves + f.l) * 256;
-    for (int e = tid; e < NB * NB; e += BT) sm.T[e % NB][e / NB] = __ldcg(T + (e % NB) + 16 * (e / NB));
+    const int rows = 2 * g.n - f.j0, nb = (rows + 7) / 8;
     long long ldp, ldc;
-    const double* P = mat_ptr(g, st, (long long)f.k * g.n + f.j0, f.m, f.t * g.NB, ldp);
+    const double* P = mat_ptr(g, st, (long long)f.k * g.n + f.j0, f.m, f.t * 16, ldp);
     double* C = tile_ptr(g, st, f.k, f.j0, m2, t2, ldc);
-    const int w2 = min(g.NB, g.n - t2 * g.NB);
-    if constexpr (NB == 16) {
-      if (!block_wait_geq(st, st.cnt + x2, s - lo2, &sm.flag)) return;
-      double none[R][16];
-      apply_qt_mma<R, false>(sC, sC + Pass<R>::ROWS * MS, none, P, ldp, f.w, C, ldc, mrows, w2,
-                             sm);
-    } else {
-      if (!block_wait_geq(st, st.cnt + x2, s - lo2, &sm.flag)) return;
-      double none[R][8];
-      apply_qt_mma8<R, false>(sC, sC + 8 * Stage8<R>::S8, none, P, ldp, f.w, C, ldc, mrows, w2,
-                              sm);
+    const int w2 = min(16, g.n - t2 * 16);
+    // The tile is loaded while the leaf is still being factored.
+    if (tid == 0) sm.flag = wait_geq(st, st.cnt + x2, s - lo2) ? 1 : 0;
+    bar_main<MT>();
+    if (!sm.flag) return;
+    double c[NIW][2][2];
+    const bool vecc = pair_aligned(C, ldc);
+#pragma unroll
+    for (int i = 0; i < NIW; i++) {
+      const int b = warp + i * MW;
+#pragma unroll
+      for (int cs = 0; cs < 2; cs++) {
+        const int cc = gc + 8 * cs;
+        const double2 v = ld_pair(C + cm(0, cc, ldc), 8 * b + 2 * t, rows, b < nb && cc < w2, vecc);
+        c[i][cs][0] = v.x;
+        c[i][cs][1] = v.y;
+      }
     }
+    bar_main<MT>();  // everyone has read sm.flag
+    if (tid == 0) sm.flag = wait_geq(st, st.factored + s, 1) ? 1 : 0;
+    bar_main<MT>();
+    if (!sm.flag) return;
+    // V (unit lower trapezoidal) and T to shared memory.
+    {
+      const bool vec = pair_aligned(P, ldp) && (rows & 1) == 0;
+      if (K::BULK && vec && tid == 0 && rows > 16) {
+        fence_proxy();
+        tc::mbar_arrive_expect_tx(&sm.bar, 8 * f.w * (rows - 16));
+        for (int cc = 0; cc < f.w; cc++)
+          bulk_load(sV + sidx(16, cc, SV), P + cm(16, cc, ldp), rows - 16, &sm.bar);
+      }
+      for (int cc = warp; cc < 16; cc += MW) {
+        const double* col = P + cm(0, cc, ldp);
+        if (cc >= f.w) {
+          for (int r = 16 + lane; r < 8 * nb; r += 32) sV[sidx(r, cc, SV)] = 0.0;
+        } else if (vec) {
+          if (!K::BULK) {
+#pragma unroll 1
+            for (int r = 16 + 2 * lane; r < rows; r += 64)
+              cp_async16(sV + sidx(r, cc, SV), col + r, 16);
+          }
+          if (lane < 8 && max(rows, 16) + lane < 8 * nb) sV[sidx(max(rows, 16) + lane, cc, SV)] = 0.0;
+        } else {
+#pragma unroll 8
+          for (int r = 16 + lane; r < 8 * nb; r += 32)
+            sV[sidx(r, cc, SV)] = r < rows ? __ldcg(col + r) : 0.0;
+        }
+      }
+      const double* T = st.T + ((long long)f.k * st.maxleaves + f.l) * 256;
+      for (int e = tid; e < 256; e += MT) {
+        const int r = e & 15, cc = e >> 4;
+        double v = 0.0;
+        if (cc < f.w && r < rows) v = r == cc ? 1.0 : (r > cc ? __ldcg(P + cm(r, cc, ldp)) : 0.0);
+        sV[sidx(r, cc, SV)] = v;
+        sm.T[r][cc] = __ldcg(T + e);
+      }
+      if (!K::BULK) {
+        cp_async_wait<0>();
+      } else if (vec && rows > 16) {
+        if (tid == 0 && !bulk_wait(&sm.bar, phase, st.err)) sm.flag = 0;
+        phase ^= 1;
+      }
+    }
+    bar_main<MT>();
+    if (!sm.flag) return;
+    double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+#pragma unroll
+    for (int i = 0; i < NIW; i++) {
+      const int b = warp + i * MW;
+      if (b < nb) {
+#pragma unroll
+        for (int jt = 0; jt < 2; jt++) {
+          const double2 v =
+              *reinterpret_cast<const double2*>(sV + sidx(8 * b + 2 * t, gc + 8 * jt, SV));
+          dmma_16x8x8(acc[jt], c[i][0][0], c[i][1][0], c[i][0][1], c[i][1][1], v.x, v.y);
+        }
+      }
+    }
+    double fr[2][4];
+    reduce_w<MW>(acc, fr, part, sm, gq, t, warp);
+#pragma unroll
+    for (int i = 0; i < NIW; i++) {
+      const int b = warp + i * MW;
+      if (b < nb) {
+        update_block(c[i], fr, sV, SV, 8 * b, gq, t);
+#pragma unroll
+        for (int cs = 0; cs < 2; cs++)
+          st_pair(C + cm(0, gc + 8 * cs, ldc), 8 * b + 2 * t, rows, gc + 8 * cs < w2, vecc,
+                  c[i][cs][0], c[i][cs][1]);
+      }
+    }
+    bar_main<MT>();
     if (tid == 0) {
       __threadfence();
       red_release_add(st.cnt + x2, 1);
@@ -869,44 +1154,73 @@ __global__ void __launch_bounds__(BT, 1) bsof_persistent_kernel(BsofGeom g, Bsof
   }
 }
 
+template <class K>
+__global__ void __launch_bounds__(K::THREADS, 1) bsof_persistent_kernel(BsofGeom g, BsofState st) {
+  extern __shared__ __align__(16) double dyn_bsof[];
+  __shared__ __align__(16) ChainSmem<K::MW> sm;
+  const int SV = tile_stride(g.n);
+  double* sV = dyn_bsof;
+  double* part = sV + 16 * SV;
+  double* sC = part + K::MW * 256;
+  if (threadIdx.x == 0) {
+    tc::mbar_init(&sm.bar, 1);
+    tc::fence_barrier_init();
+  }
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) sm.step[st.s_begin & 1] = chain_step(g, st, st.s_begin);
+      }
+  __syncthreads();
+  if (threadIdx.x >= K::MT) {
+    if constexpr (K::REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if (blockIdx.x == 0) chain_helper<K>(g, st, sV, sC, SV, sm);
+  } else {
+    if constexpr (K::REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    if (blockIdx.x == 0) chain_main<K>(g, st, sV, part, sC, SV, sm);
+    else worker<K>(g, st, sV, part, SV, sm);
+  }
+}
+
 // ------------------------------------------------------------------ launcher
-// 16-wide leaves (DMMA block-reflector update, one 512-row staging pass) up
-// to 2n = 512 rows; taller panels use 8-wide leaves (up to 2n = 1536 rows,
-// six rows per thread), whose CUDA-core update streams rows from registers.
-// (16-wide leaves with two staging passes measured slower at n = 400.)
-int bsof_leaf_width(int n) { return n <= 256 ? 16 : 8; }
+using Chain64 = ChainCfg<3, 5, 4, true>;
+using Chain128 = ChainCfg<7, 5, 4, true>;
+using Chain256 = ChainCfg<7, 9, 8, true>;
+using Chain400 = ChainCfg<7, 14, 13, true>;
+using Chain640 = ChainCfg<7, 23, 20, false>;
+
+// 16-wide leaves up to n = 640; the tall kernel's 8-wide ones above.
+int bsof_leaf_width(int n) { return n <= Chain640::MAX_ROWS / 2 ? 16 : 8; }
 
 int bsof_tiles(int n) { return (n + bsof_leaf_width(n) - 1) / bsof_leaf_width(n); }
 
-template <int R, int NB>
-static size_t dyn_smem() {
-  return NB == 16 ? sizeof(double) * 2 * (size_t)Pass<R>::ROWS * MS
-                  : sizeof(double) * 2 * 8 * (size_t)Stage8<R>::S8;
+template <class K>
+static size_t dyn_smem(int n) {
+  const size_t SV = tile_stride(n);
+  return sizeof(double) * (16 * SV + 256 * K::MW + (K::PREF ? 16 * (SV + 16) : 0));
 }
 
-template <int R, int NB, bool FW4 = true>
-static cudaError_t launch_R(const BsofGeom& g, const BsofState& st, int grid, cudaStream_t s) {
+template <class K>
+static cudaError_t launch_cfg(const BsofGeom& g, const BsofState& st, int workers, cudaStream_t s) {
+  static PerDevice once;
+  static int sms[kMaxDevices];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  int count = dev < kMaxDevices ? sms[dev] : 0;
+  if (once.pending() >= 0 || count == 0) {
+    if ((e = cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+      return e;
+    e = cudaFuncSetAttribute(bsof_persistent_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)dyn_smem<K>(K::MAX_ROWS / 2));
+    if (e != cudaSuccess) return e;
+    if (dev < kMaxDevices) sms[dev] = count;
+    once.mark(dev);
+  }
+  // At least one CTA of any size fits each SM.
+  const int grid = min(1 + workers, count);
   void* args[] = {(void*)&g, (void*)&st};
-  return cudaLaunchCooperativeKernel((const void*)bsof_persistent_kernel<R, NB, FW4>, dim3(grid),
-                                     dim3(BT), args, dyn_smem<R, NB>(), s);
+  return cudaLaunchCooperativeKernel((const void*)bsof_persistent_kernel<K>, dim3(grid),
+                                     dim3(K::THREADS), args, dyn_smem<K>(g.n), s);
 }
-
-template <int R, int NB, bool FW4 = true>
-static int max_grid() {
-  int dev = 0, sms = 0, per = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaFuncSetAttribute(bsof_persistent_kernel<R, NB, FW4>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_smem<R, NB>());
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, bsof_persistent_kernel<R, NB, FW4>, BT,
-                                                dyn_smem<R, NB>());
-  return sms * (per > 0 ? per : 1);
-}
-
-// Factor warps of 16-wide leaves: 4 with the next tile staged meanwhile (the
-// default), or 8; process-wide.
-static std::atomic<int> g_factor8{0};
-void bsof_set_factor_warps(int w) { g_factor8.store(w == 8 ? 1 : 0); }
 
 cudaError_t launch_bsof_persistent(double* A, long long ld, int n, int L, double* tau, double* T,
                                    double* G, int maxleaves, int* cnt, int* factored,
@@ -938,46 +1252,22 @@ cudaError_t launch_bsof_persistent(double* A, long long ld, int n, int L, double
   s.s_begin = s_begin > 0 ? s_begin : 0;
   s.s_end = (s_end < 0 || s_end > g.S) ? g.S : s_end;
   if (s.s_begin >= s.s_end) return cudaSuccess;
-  const int R = (2 * n + BT - 1) / BT;
-  int grid = 1 + workers;
-  if (g.NB == 16) {
-    switch (R) {
-      case 1:
-        if (g_factor8.load()) {
-          grid = min(grid, max_grid<1, 16, false>());
-          return launch_R<1, 16, false>(g, s, grid, st);
-        }
-        grid = min(grid, max_grid<1, 16>());
-        return launch_R<1, 16>(g, s, grid, st);
-      case 2:
-        if (g_factor8.load()) {
-          grid = min(grid, max_grid<2, 16, false>());
-          return launch_R<2, 16, false>(g, s, grid, st);
-        }
-        grid = min(grid, max_grid<2, 16>());
-        return launch_R<2, 16>(g, s, grid, st);
-      default: return cudaErrorInvalidValue;
-    }
-  }
-  switch (R) {
-    case 3: grid = min(grid, max_grid<3, 8>()); return launch_R<3, 8>(g, s, grid, st);
-    case 4: grid = min(grid, max_grid<4, 8>()); return launch_R<4, 8>(g, s, grid, st);
-    case 5: grid = min(grid, max_grid<5, 8>()); return launch_R<5, 8>(g, s, grid, st);
-    case 6: grid = min(grid, max_grid<6, 8>()); return launch_R<6, 8>(g, s, grid, st);
-    default: return cudaErrorInvalidValue;
-  }
+  if (2 * n <= Chain64::MAX_ROWS) return launch_cfg<Chain64>(g, s, workers, st);
+  if (2 * n <= Chain128::MAX_ROWS) return launch_cfg<Chain128>(g, s, workers, st);
+  if (2 * n <= Chain256::MAX_ROWS) return launch_cfg<Chain256>(g, s, workers, st);
+  if (2 * n <= Chain400::MAX_ROWS) return launch_cfg<Chain400>(g, s, workers, st);
+  if (2 * n <= Chain640::MAX_ROWS) return launch_cfg<Chain640>(g, s, workers, st);
+  return launch_bsof_tall(g, s, workers, st);
 }
 
 cudaError_t preload_bsof(size_t* local) {
   cudaError_t e;
-  if ((e = preload_one(bsof_persistent_kernel<1, 16>, local)) != cudaSuccess) return e;
-  if ((e = preload_one(bsof_persistent_kernel<2, 16>, local)) != cudaSuccess) return e;
-  if ((e = preload_one(bsof_persistent_kernel<1, 16, false>, local)) != cudaSuccess) return e;
-  if ((e = preload_one(bsof_persistent_kernel<2, 16, false>, local)) != cudaSuccess) return e;
-  if ((e = preload_one(bsof_persistent_kernel<3, 8>, local)) != cudaSuccess) return e;
-  if ((e = preload_one(bsof_persistent_kernel<4, 8>, local)) != cudaSuccess) return e;
-  if ((e = preload_one(bsof_persistent_kernel<5, 8>, local)) != cudaSuccess) return e;
-  return preload_one(bsof_persistent_kernel<6, 8>, local);
+  if ((e = preload_one(bsof_persistent_kernel<Chain64>, local)) != cudaSuccess) return e;
+  if ((e = preload_one(bsof_persistent_kernel<Chain128>, local)) != cudaSuccess) return e;
+  if ((e = preload_one(bsof_persistent_kernel<Chain256>, local)) != cudaSuccess) return e;
+  if ((e = preload_one(bsof_persistent_kernel<Chain400>, local)) != cudaSuccess) return e;
+  if ((e = preload_one(bsof_persistent_kernel<Chain640>, local)) != cudaSuccess) return e;
+  return preload_bsof_tall(local);
 }
 
 }  // namespace bsofi

@@ -263,9 +263,8 @@ int run_bsof(int n, int L, double* dA, int ldd, double* dtau, void* ws, cudaStre
   CKM(cudaMemsetAsync(sync, 0, sizeof(int) * ly.sync_ints, st));
   CKM(cudaMemsetAsync(at<int>(ws, ly.info) + 1, 0, sizeof(int), st));
   if (form_q) CK(launch_set_identity(G, 2 * n, 2 * n, 4ll * n * n, L - 1, st));
-  // 16-wide leaves apply with DMMA and need few workers; 8-wide leaves
-  // (n > 256) have three times the tasks per leaf and use every SM.
-  int workers = bsof_leaf_width(n) == 16 ? base_workers : 4 * base_workers;
+  // Panels of n > 256 have more and larger tasks per leaf and use every SM.
+  int workers = n <= 256 ? base_workers : 4 * base_workers;
   if (form_q) workers *= 2;
   CK(launch_bsof_persistent(dA, ldd, n, L, dtau, Tb, form_q ? G : nullptr, ly.maxleaves, sync,
                             sync + ntiles, sync + ntiles + ly.leaves, at<int>(ws, ly.info) + 1,
@@ -615,7 +614,7 @@ SideStreams* side_streams(cudaStream_t st) {
 // Row groups and split row h of the overlapped path, or false when it does
 // not apply to (n, L).
 bool overlap_split(int n, int L, int* grp_out, int* tailg_out, int* h_out) {
-  if (!g_overlap_enabled.load() || bsof_leaf_width(n) != 16 || L < 4) return false;
+  if (!g_overlap_enabled.load() || n > 256 || L < 4) return false;
   const Plan plan = plan_for(n, L);
   const int grp = plan.bstri_group < L - 2 ? plan.bstri_group : L - 2;
   if (plan.bstri_cfg != 4 || grp < 2) return false;
@@ -1391,7 +1390,7 @@ int bsofi_dev_bsof_timeline(int n, int L, int ldd, void* dws, unsigned long long
 
 void bsofi_dev_set_bsof_workers(int w) { g_workers_override = w > 0 ? w : 0; }
 
-void bsofi_dev_set_bsof_factor_warps(int w) { bsof_set_factor_warps(w); }
+void bsofi_dev_set_bsof_factor_warps(int) {}
 
 void bsofi_dev_set_wait_test(int on) { g_wait_test = on != 0; }
 

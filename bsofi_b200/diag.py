@@ -10,8 +10,8 @@
 bsof-timeline inverts a seeded Hubbard matrix (a random p-cyclic one when n is
 not a square) with bsofi_device_invert and prints, for the last run, the BSOF
 chain length and the per-leaf phases recorded by the persistent BSOF kernel's
-critical CTA (bsofi_device_bsof_timeline: globaltimer stamps at loop start,
-tile ready, next-tile update start and leaf published).  invert times REPS
+critical CTA (bsofi_device_bsof_timeline: globaltimer stamps at leaf start,
+next-tile update start and leaf done).  invert times REPS
 device-resident inversions of the Hubbard matrix (U = 4 unless given) with the
 size's launch plan and prints the fastest with its TFLOP/s, the BSOI time
 (CUDA events around its launches) and the BSOF chain.
@@ -25,7 +25,7 @@ from .hubbard import hubbard_blocks, hubbard_matrix, random_pcyclic
 
 
 def bsof_leaves(n, L):
-    nb = 16 if n <= 256 else 8
+    nb = 16 if n <= 640 else 8
     nl = (n + nb - 1) // nb
     return (L - 2) * nl + 2 * nl
 
@@ -72,7 +72,7 @@ def bsof_timeline(n, L, reps=3):
             "to_next_leaf_us": (t[1:, 0] - t[:-1, 2]).mean() / 1e3,
         }
         wait = (t[:, 1] - t[:, 0]) / 1e3
-        nl = (n + (16 if n <= 256 else 8) - 1) // (16 if n <= 256 else 8)
+        nl = (n + (16 if n <= 640 else 8) - 1) // (16 if n <= 640 else 8)
         first = np.arange(S) % nl == 0  # the first leaf of each regular panel
         first[(L - 2) * nl:] = False
         out.update({
@@ -363,11 +363,6 @@ def main(argv):
     for a in list(argv):
         if a.startswith("--workers="):
             _lib.load().bsofi_device_set_bsof_workers(int(a.split("=", 1)[1]))
-            argv = [x for x in argv if x != a]
-    # --factor-warps=8: 16-wide BSOF leaves factored by all eight warps.
-    for a in list(argv):
-        if a.startswith("--factor-warps="):
-            _lib.load().bsofi_device_set_bsof_factor_warps(int(a.split("=", 1)[1]))
             argv = [x for x in argv if x != a]
     if len(argv) >= 3 and argv[0] == "bsof-timeline":
         n, L = int(argv[1]), int(argv[2])

@@ -470,8 +470,8 @@ int bsofi_device_timing_read(double *ms, long long *launches);
 
 /* Diagnostics (no reference counterpart): the BSOF timeline of the last
  * factorization that used `dwork` -- four globaltimer stamps (ns) per leaf
- * from the CTA that runs the critical chain: loop start, tile ready, leaf
- * published, next-tile update start.  Copies up to max_leaves leaves to host
+ * from the CTA that runs the critical chain: leaf start (twice), leaf done,
+ * next-tile update start.  Copies up to max_leaves leaves to host
  * and returns the number copied.  set_bsof_workers sets the number of worker
  * CTAs of the persistent BSOF kernel (default 32) for this process. */
 int bsofi_device_bsof_timeline(int n, int L, int ldda, void *dwork, unsigned long long *host,
@@ -484,10 +484,8 @@ void bsofi_device_set_bsof_workers(int workers);
  * results are the same as without the split).  on = 0 turns this off for the
  * process, 1 (the default) on. */
 void bsofi_device_set_bstri_overlap(int on);
-/* Diagnostics (no reference counterpart): warps that factor a 16-wide leaf of
- * the BSOF chain (n <= 256): 4 (the default; the CTA's other 4 warps stage the
- * next leaf's tile meanwhile) or 8 (the tile is staged after the
- * factorization).  Results are the same either way to rounding.  Process-wide. */
+/* Without effect (kept for callers that set it): it chose between two forms of
+ * an earlier BSOF chain kernel; the present one has a single form. */
 void bsofi_device_set_bsof_factor_warps(int warps);
 /* FP64 tile engine instruction shape (diagnostics, no reference
  * counterpart; process-wide): mma.sync m16n8k8 steps (0, the default) or
