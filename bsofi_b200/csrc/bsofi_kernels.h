@@ -72,6 +72,12 @@ cudaError_t launch_bstri_recurrence_blocked(double* A, long long ld, const doubl
                                             int* done, int* next, int* err, cudaStream_t st,
                                             int hfloor = 0);
 
+// BSTRI's recurrence for n <= 128 as one launch of column bands
+// (kernels_bstri_band.cu): W packed, the diagonal blocks of A inverted, Z in
+// block column L-1.
+cudaError_t launch_bstri_band(double* A, long long ld, const double* W, int n, int L,
+                              cudaStream_t st);
+
 // Persistent BSOI (kernels_bsoi.cu): all p-1 steps in one launch.
 // done: (L-1) * bsoi_row_bands(N) ints and next: one int, zeroed before;
 // small: 64 x 64 tiles instead of 128 x 128.  never (diagnostics): a zeroed
@@ -84,6 +90,13 @@ cudaError_t launch_bsoi_persistent(double* A, long long ld, double* carry0, doub
                                    long long ldc, const double* G, int n, int L, int* done,
                                    int* next, int* err, bool small, cudaStream_t st,
                                    int row0 = 0, int row1 = -1, const int* never = nullptr);
+
+// BSOI of small blocks as one launch of row bands (kernels_bsoi_band.cu),
+// carry seed and X(:,0) included; the info words {info, BSOF error, BSOI error,
+// BSTRI error} are folded as by launch_copy_masked.  Only where bsoi_band_fits.
+bool bsoi_band_fits(int n, int L);
+cudaError_t launch_bsoi_band(double* A, long long ld, const double* G, int n, int L, int* info,
+                             cudaStream_t st);
 
 // BSOI of many instances in one persistent launch (kernels_bsoi.cu).  Each
 // instance: its matrix, carries, G_k, sizes, its done counters ((L-1) *
@@ -190,7 +203,9 @@ cudaError_t launch_ozaki_product(const OzProduct& p, cudaStream_t st);
 // One per kernel file: every kernel (each template instance) it launches.
 cudaError_t preload_bsof(size_t* local);
 cudaError_t preload_bsoi(size_t* local);
+cudaError_t preload_bsoi_band(size_t* local);
 cudaError_t preload_bstri(size_t* local);
+cudaError_t preload_bstri_band(size_t* local);
 cudaError_t preload_gemm(size_t* local);
 cudaError_t preload_panel(size_t* local);
 cudaError_t preload_tri(size_t* local);

@@ -104,13 +104,14 @@ Plan default_plan(int n, int L) {
 // another instance's cooperative BSOF launch could not start meanwhile.
 thread_local bool g_nonpersistent = false;
 
+Plan stored_plan(int n, int L) {
+  std::lock_guard<std::mutex> lk(g_plan_mu);
+  auto it = g_plans.find({n, L});
+  return it == g_plans.end() ? default_plan(n, L) : it->second;
+}
+
 Plan plan_for(int n, int L) {
-  Plan p;
-  {
-    std::lock_guard<std::mutex> lk(g_plan_mu);
-    auto it = g_plans.find({n, L});
-    p = it == g_plans.end() ? default_plan(n, L) : it->second;
-  }
+  Plan p = stored_plan(n, L);
   if (g_nonpersistent) {
     if (p.bsoi == 0) p.bsoi = 3;  // per-step 128 x 128 (K stage 32)
     if (p.bsoi == 5) p.bsoi = 2;  // per-step 64 x 64
@@ -125,6 +126,29 @@ thread_local int g_workers_override = 0;
 // nothing writes (the spare int after the BSOI tile counter), so their
 // bounded waits give up.
 thread_local bool g_wait_test = false;
+
+// Whether BSOI runs as one launch of row bands (kernels_bsoi_band.cu) and
+// BSTRI's recurrence as one of column bands (kernels_bstri_band.cu): blocks of
+// at most 128 with row bands of at most 64 rows, one per SM, where the plan's
+// knob is the size's default (a tuned plan that chose another form keeps it).
+// In pipelined batches only where the launches are short (a long one would
+// keep the next chains' launches waiting).
+bool band_size(int n, int L) {
+  if (g_nonpersistent && n * L > 2400) return false;
+  return bsoi_band_fits(n, L);
+}
+
+bool use_bsoi_band(int n, int L) {
+  if (g_wait_test || !band_size(n, L)) return false;
+  const Plan p = stored_plan(n, L), d = default_plan(n, L);
+  return p.bsoi == d.bsoi && (p.bsoi == 1 || p.bsoi == 5);
+}
+
+bool use_bstri_band(int n, int L) {
+  if (!band_size(n, L)) return false;
+  const Plan p = stored_plan(n, L), d = default_plan(n, L);
+  return p.bstri_cfg == d.bstri_cfg && p.bstri_group == d.bstri_group;
+}
 
 // Worker CTAs of one BSOF launch: the caller's count, else the override, else
 // the plan's.
@@ -512,6 +536,11 @@ int run_bstri(int n, int L, double* dA, int ldd, void* ws, cudaStream_t st) {
   double* last = dA + cm(0, (long long)(L - 1) * n, ldd);
   if (int e = yz_products(n, L, dA, ldd, last, ldd, Y, st)) return e;
   if (int e = w_products(n, dA, ldd, W, 0, L - 2, st)) return e;
+  if (use_bstri_band(n, L)) {
+    CKM(cudaMemsetAsync(info + 3, 0, sizeof(int), st));
+    CK(launch_bstri_band(dA, ldd, W, n, L, st));
+    return 0;
+  }
   // Row recurrence: X_{i, i+1:L} = W_i X_{i+1, i+1:L} (+ Z_i on the last block).
   const Plan plan = plan_for(n, L);
   const int rec = plan.bstri_cfg;
@@ -614,7 +643,7 @@ SideStreams* side_streams(cudaStream_t st) {
 // Row groups and split row h of the overlapped path, or false when it does
 // not apply to (n, L).
 bool overlap_split(int n, int L, int* grp_out, int* tailg_out, int* h_out) {
-  if (!g_overlap_enabled.load() || n > 256 || L < 4) return false;
+  if (!g_overlap_enabled.load() || n > 256 || L < 4 || use_bstri_band(n, L)) return false;
   const Plan plan = plan_for(n, L);
   const int grp = plan.bstri_group < L - 2 ? plan.bstri_group : L - 2;
   if (plan.bstri_cfg != 4 || grp < 2) return false;
@@ -883,6 +912,12 @@ int run_bsoi(int n, int L, double* dA, int ldd, const double* dtau, void* ws, cu
   if (!q_ready) {
     int e = bsoi_form_q(n, L, dA, ldd, dtau, ws, st);
     if (e) return e;
+  }
+  if (use_bsoi_band(n, L)) {
+    if (g_timer.on) CKM(g_timer.mark(st));
+    CK(launch_bsoi_band(dA, ldd, G, n, L, at<int>(ws, ly.info), st));
+    if (g_timer.on) CKM(g_timer.mark(st));
+    return 0;
   }
   int e = bsoi_carry(n, L, dA, ldd, ws, st);
   if (e) return e;
@@ -1240,7 +1275,9 @@ int bsofi_dev_preload(void) {
   if ((e = gemm_init_attributes()) != cudaSuccess) return (int)e;
   if ((e = preload_bsof(&local)) != cudaSuccess) return (int)e;
   if ((e = preload_bsoi(&local)) != cudaSuccess) return (int)e;
+  if ((e = preload_bsoi_band(&local)) != cudaSuccess) return (int)e;
   if ((e = preload_bstri(&local)) != cudaSuccess) return (int)e;
+  if ((e = preload_bstri_band(&local)) != cudaSuccess) return (int)e;
   if ((e = preload_gemm(&local)) != cudaSuccess) return (int)e;
   if ((e = preload_panel(&local)) != cudaSuccess) return (int)e;
   if ((e = preload_tri(&local)) != cudaSuccess) return (int)e;
