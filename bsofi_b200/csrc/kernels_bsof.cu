@@ -59,23 +59,18 @@
 
 namespace bsofi {
 
-// FW row warps of NI 8-row blocks each, one top warp, helper warps.  PREF:
-// the next tile fits in shared memory beside V and is staged there by the
-// helper warps while the leaf is factored.  NIW: 8-row blocks per warp of a
-// worker (all FW + 1 warps take rows there).
-template <int FW_, int NI_, int NIW_, bool PREF_>
+// FW row warps of NI 8-row blocks each, one top warp, helper warps (which
+// stage the next tile in shared memory beside V while the leaf is factored).
+// NIW: 8-row blocks per warp of a worker (all FW + 1 warps take rows there).
+template <int FW_, int NI_, int NIW_>
 struct ChainCfg {
   static constexpr int FW = FW_, NI = NI_, NIW = NIW_;
-  static constexpr bool PREF = PREF_;
   static constexpr int MW = FW + 1, MT = 32 * MW;
-  static constexpr int HW = 4;
+  static constexpr int HW = 4;  // helper warps: one builds T, the others load and store
   static constexpr int THREADS = MT + 32 * HW;
   static constexpr int CT = MT + 32;  // column barrier: with the T warp, the last helper
   // Row slots are taken in groups of GS, skipped when every row is finished.
   static constexpr int GS = 3, NG = (NI + GS - 1) / GS;
-  // The pivot column's shuffled values are kept from the dot products to the
-  // update where registers allow, else shuffled again.
-  static constexpr bool KEEPX = NI <= 14;
   // Tiles move between global and shared memory by bulk copies, which keep the
   // load/store pipe free for the computing warps, or (short panels, where the
   // chain waits for the workers' answer and latency counts) by cp.async and
@@ -357,8 +352,8 @@ BSOFI_DEVINL void put_partials(double* red, double d0, double d1, int g, int t, 
 // the next pivot column J = I+1 (half CSD).  ab8: first 8-row block of the
 // leaf; nb: row blocks of the panel.
 template <class K, bool UPD0, int CSU, int CSD>
-BSOFI_DEVINL void row_pass(double (&a)[K::NI][2][2], double (&x)[K::KEEPX ? K::NI : 1][2],
-                           double f0, double f1, int srcu, int srcd, int ab8, int nb, int warp,
+BSOFI_DEVINL void row_pass(double (&a)[K::NI][2][2], double (&x)[K::NI][2],
+                           double f0, double f1, int srcd, int ab8, int nb, int warp,
                            double& d0, double& d1) {
   double s0[2] = {0.0, 0.0}, s1[2] = {0.0, 0.0};
 #pragma unroll
@@ -370,13 +365,11 @@ BSOFI_DEVINL void row_pass(double (&a)[K::NI][2][2], double (&x)[K::KEEPX ? K::N
     for (int i = ia; i < ie; i++) {
 #pragma unroll
       for (int h = 0; h < 2; h++) {
-        double xo;
-        if constexpr (K::KEEPX) xo = x[i][h];
-        else xo = shfl_d(a[i][CSU][h], srcu);
+        const double xo = x[i][h];
         if (UPD0) a[i][0][h] = fma(-xo, f0, a[i][0][h]);
         a[i][1][h] = fma(-xo, f1, a[i][1][h]);
         const double xn = shfl_d(a[i][CSD][h], srcd);
-        if constexpr (K::KEEPX) x[i][h] = xn;
+        x[i][h] = xn;
         s0[h] = fma(xn, a[i][0][h], s0[h]);
         s1[h] = fma(xn, a[i][1][h], s1[h]);
       }
@@ -388,7 +381,7 @@ BSOFI_DEVINL void row_pass(double (&a)[K::NI][2][2], double (&x)[K::KEEPX ? K::N
 
 // The dot products with column 0, before the first column step.
 template <class K>
-BSOFI_DEVINL void row_first(double (&a)[K::NI][2][2], double (&x)[K::KEEPX ? K::NI : 1][2], int t,
+BSOFI_DEVINL void row_first(double (&a)[K::NI][2][2], double (&x)[K::NI][2], int t,
                             double& d0, double& d1) {
   double s0[2] = {0.0, 0.0}, s1[2] = {0.0, 0.0};
 #pragma unroll
@@ -396,7 +389,7 @@ BSOFI_DEVINL void row_first(double (&a)[K::NI][2][2], double (&x)[K::KEEPX ? K::
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       const double xn = shfl_d(a[i][0][h], t);
-      if constexpr (K::KEEPX) x[i][h] = xn;
+      x[i][h] = xn;
       s0[h] = fma(xn, a[i][0][h], s0[h]);
       s1[h] = fma(xn, a[i][1][h], s1[h]);
     }
@@ -430,7 +423,7 @@ BSOFI_DEVINL void factor_rows(double (&a)[K::NI][2][2], ChainSmem<K::MW>& sm, in
                               int nb, int g, int t, int warp) {
   constexpr int MW = K::MW;
   const int c0 = col_of(g), c1 = c0 + 8;
-  double x[K::KEEPX ? K::NI : 1][2];
+  double x[K::NI][2];
   double d0, d1;
   row_first<K>(a, x, t, d0, d1);
   put_partials<MW>(sm.red[0], d0, d1, g, t, warp);
@@ -439,9 +432,8 @@ BSOFI_DEVINL void factor_rows(double (&a)[K::NI][2][2], ChainSmem<K::MW>& sm, in
     bar_col<K::CT>();
     const ColStep c = col_step<MW>(sm, I, g, t);
     const double f0 = c0 > I ? c.rf.q * c.w0 : 0.0, f1 = c1 > I ? c.rf.q * c.w1 : 0.0;
-    const int su = group_of(I & 7) * 4 + t, sd = group_of((I + 1) & 7) * 4 + t;
-    row_pass<K, upd0.value != 0, csu.value, csd.value>(a, x, f0, f1, su, sd, ab8, nb, warp, d0,
-                                                       d1);
+    const int sd = group_of((I + 1) & 7) * 4 + t;
+    row_pass<K, upd0.value != 0, csu.value, csd.value>(a, x, f0, f1, sd, ab8, nb, warp, d0, d1);
     put_partials<MW>(sm.red[(I + 1) & 1], d0, d1, g, t, warp);
   };
   using Z = std::integral_constant<int, 0>;
@@ -641,7 +633,7 @@ BSOFI_DEVINL void update_block(double (&c)[2][2], const double (&fr)[2][4], cons
 }
 
 // ------------------------------------------------------------ the chain CTA
-// The helper warps: wait for the next tile and (PREF) stage it while the leaf
+// The helper warps: wait for the next tile and stage it while the leaf
 // is being factored, build T; store and publish the leaf while the next tile
 // is being updated.
 template <class K>
@@ -672,7 +664,6 @@ BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const dou
       bar_all<K::THREADS>();
       if (!sm.flag) return;
       if (lane == 0 && s + 1 < st.s_end) sm.step[(s + 1) & 1] = chain_step(g, st, s + 1);
-      if (!K::PREF && sm.step[s & 1].trans) bar_all<K::THREADS>();
       bar_all<K::THREADS>();
     }
     return;
@@ -681,7 +672,7 @@ BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const dou
     const ChainStep& z = sm.step[s & 1];
     if (ht == 0)
       sm.flag = !z.next || wait_geq(st, st.cnt + tile_id(g, z.m2, z.t2), s - z.lo2) ? 1 : 0;
-    if constexpr (K::PREF) {
+    {
       bar_help<32 * LW>();
       if (z.next && sm.flag) {
         // Rows [ab, rows) of the tile, then (fresh) the n rows below the panel
@@ -769,7 +760,6 @@ BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const dou
       __threadfence();
       red_release_add(st.factored + s, 1);
     }
-    if (!K::PREF && z.trans) bar_all<K::THREADS>();  // V may be overwritten
     bar_all<K::THREADS>();
   }
 }
@@ -893,11 +883,7 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
           for (int cs = 0; cs < 2; cs++) {
             const int cc = gc + 8 * cs;
             double2 v = make_double2(0.0, 0.0);
-            if constexpr (K::PREF) {
-              if (live) v = *reinterpret_cast<const double2*>(sC + sidx(r, cc, SC));
-            } else {
-              v = ld_pair(C + cm(0, cc, ldc), r, rows, live && cc < w2, vec);
-            }
+            if (live) v = *reinterpret_cast<const double2*>(sC + sidx(r, cc, SC));
             c[i][cs][0] = v.x;
             c[i][cs][1] = v.y;
           }
@@ -962,18 +948,14 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
           }
         }
       } else {
-        // Through shared memory: over the tile just read (PREF), else over V
-        // once the helpers have stored it.
-        double* sX = K::PREF ? sC : sV;
-        const int SX = K::PREF ? SC : SV;
-        if constexpr (!K::PREF) bar_all<K::THREADS>();
+        // Through shared memory, over the tile just read.
 #pragma unroll
         for (int i = 0; i < NI; i++) {
           const int b = bb + i * bs;
           if (b < blo || b >= bhi) continue;
 #pragma unroll
           for (int cs = 0; cs < 2; cs++)
-            *reinterpret_cast<double2*>(sX + sidx(8 * b + 2 * t, gc + 8 * cs, SX)) =
+            *reinterpret_cast<double2*>(sC + sidx(8 * b + 2 * t, gc + 8 * cs, SC)) =
                 make_double2(c[i][cs][0], c[i][cs][1]);
         }
         bar_main<MT>();
@@ -989,13 +971,11 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
               double v = 0.0;
               if ((!top || i < 2) && r < rows2 && cc < w2) {
                 if (r < n) {
-                  v = sX[sidx(n + r, cc, SX)];
-                } else if constexpr (K::PREF) {
+                  v = sC[sidx(n + r, cc, SC)];
+                } else {
                   int rr = 8 * nb + r - n;
                   if (rr >= capc) rr -= capc;
                   v = sC[sidx(rr, cc, SC)];
-                } else {
-                  v = __ldcg(C + cm(n + r, cc, ldc));
                 }
               }
               a[i][cs][h] = v;
@@ -1181,21 +1161,21 @@ __global__ void __launch_bounds__(K::THREADS, 1) bsof_persistent_kernel(BsofGeom
 }
 
 // ------------------------------------------------------------------ launcher
-using Chain64 = ChainCfg<3, 5, 4, true>;
-using Chain128 = ChainCfg<7, 5, 4, true>;
-using Chain256 = ChainCfg<7, 9, 8, true>;
-using Chain400 = ChainCfg<7, 14, 13, true>;
-using Chain640 = ChainCfg<7, 23, 20, false>;
+using Chain64 = ChainCfg<3, 5, 4>;
+using Chain128 = ChainCfg<7, 5, 4>;
+using Chain256 = ChainCfg<7, 9, 8>;
+using Chain400 = ChainCfg<7, 14, 13>;
 
-// 16-wide leaves up to n = 640; the tall kernel's 8-wide ones above.
-int bsof_leaf_width(int n) { return n <= Chain640::MAX_ROWS / 2 ? 16 : 8; }
+// 16-wide leaves up to n = 400, where the next tile still fits in shared
+// memory beside V; the tall kernel's 8-wide ones above.
+int bsof_leaf_width(int n) { return n <= Chain400::MAX_ROWS / 2 ? 16 : 8; }
 
 int bsof_tiles(int n) { return (n + bsof_leaf_width(n) - 1) / bsof_leaf_width(n); }
 
 template <class K>
 static size_t dyn_smem(int n) {
   const size_t SV = tile_stride(n);
-  return sizeof(double) * (16 * SV + 256 * K::MW + (K::PREF ? 16 * (SV + 16) : 0));
+  return sizeof(double) * (16 * SV + 256 * K::MW + 16 * (SV + 16));
 }
 
 template <class K>
@@ -1256,7 +1236,6 @@ cudaError_t launch_bsof_persistent(double* A, long long ld, int n, int L, double
   if (2 * n <= Chain128::MAX_ROWS) return launch_cfg<Chain128>(g, s, workers, st);
   if (2 * n <= Chain256::MAX_ROWS) return launch_cfg<Chain256>(g, s, workers, st);
   if (2 * n <= Chain400::MAX_ROWS) return launch_cfg<Chain400>(g, s, workers, st);
-  if (2 * n <= Chain640::MAX_ROWS) return launch_cfg<Chain640>(g, s, workers, st);
   return launch_bsof_tall(g, s, workers, st);
 }
 
@@ -1266,7 +1245,6 @@ cudaError_t preload_bsof(size_t* local) {
   if ((e = preload_one(bsof_persistent_kernel<Chain128>, local)) != cudaSuccess) return e;
   if ((e = preload_one(bsof_persistent_kernel<Chain256>, local)) != cudaSuccess) return e;
   if ((e = preload_one(bsof_persistent_kernel<Chain400>, local)) != cudaSuccess) return e;
-  if ((e = preload_one(bsof_persistent_kernel<Chain640>, local)) != cudaSuccess) return e;
   return preload_bsof_tall(local);
 }
 

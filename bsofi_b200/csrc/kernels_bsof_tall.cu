@@ -1,6 +1,9 @@
 // BSOF for the tallest panels (n above the 16-wide leaves' limit, up to 768):
 // the schedule of kernels_bsof.cu with 8-wide leaves, so that 1536 rows fit
-// the registers of one CTA (six rows of eight columns a thread).
+// the registers of one CTA (TR = 4, 5 or 6 rows of eight columns a thread).
+// 16-wide leaves of that height leave no room to stage the next tile and spill
+// (n = 576, p = 12: 15.7 against 16.0 ms, but slower below: an inversion at
+// n = 450, p = 3 took 5.7 against 4.0 ms), so they end at n = 400.
 #include <climits>
 #include "bsof_sched.cuh"
 #include "bsofi_kernels.h"
@@ -11,7 +14,6 @@ namespace {
 constexpr int BT = 256;  // threads per CTA
 constexpr int BW = BT / 32;
 constexpr int NB = 8;   // leaf width
-constexpr int TR = 6;   // rows per thread: panels of up to 1536 rows
 
 // Sum NB values per lane over a warp (transpose reduction): lane l ends with
 // the warp sum of value (l >> 2) & 7.
@@ -77,6 +79,7 @@ BSOFI_DEVINL void t_column(Smem& sm, int I, int lane) {
 // product d_c = sum_{r>I} a_rI a_rc with a pending column (position 0 gives
 // ||x||^2) or e_j = sum_{r>I} v_j[r] a_rI with a finished reflector, which
 // builds the dlarft factor T(0:I,I) = -tau_I T(0:I,0:I) V^T v_I.
+template <int TR>
 BSOFI_DEVINL void factor_leaf(double (&a)[TR][NB], Smem& sm, int m, int w, double* tau_out) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int SH = 2;
@@ -193,13 +196,16 @@ BSOFI_DEVINL void factor_leaf(double (&a)[TR][NB], Smem& sm, int m, int w, doubl
 // both products are free of bank conflicts.  VREG: V comes from the factoring
 // CTA's registers (thread t owns rows t + BT*i), else from the stored leaf.
 // wv: width of the leaf, w: width of the target tile.
-constexpr int S8 = TR * BT + 4;
+template <int TR>
+struct Stage8 {
+  static constexpr int S8 = TR * BT + 4;
+};
 
-template <bool VREG>
+template <int TR, bool VREG>
 BSOFI_DEVINL void apply_qt_mma8(double* sV, double* sC, const double (&a)[TR][8],
                                 const double* P, long long ldp, int wv, double* C, long long ld,
                                 int m, int w, Smem& sm) {
-  constexpr int KW = TR * BT / BW;
+  constexpr int S8 = Stage8<TR>::S8, KW = TR * BT / BW;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
@@ -263,7 +269,9 @@ BSOFI_DEVINL void apply_qt_mma8(double* sV, double* sC, const double (&a)[TR][8]
   __syncthreads();
 }
 
+template <int TR>
 __global__ void __launch_bounds__(BT, 1) bsof_tall_kernel(BsofGeom g, BsofState st) {
+  constexpr int S8 = Stage8<TR>::S8;
   __shared__ Smem sm;
   extern __shared__ __align__(16) double sC[];  // V and C tiles, 8 columns of S8 each
   const int tid = threadIdx.x;
@@ -310,7 +318,7 @@ __global__ void __launch_bounds__(BT, 1) bsof_tall_kernel(BsofGeom g, BsofState 
         for (int c = 0; c < NB; c++)
           a[i][c] = (r < mrows && c < f.w) ? __ldcg(P + cm(r, c, ldp)) : 0.0;
       }
-      factor_leaf(a, sm, mrows, f.w, st.tau + (long long)f.k * g.n + f.j0);
+      factor_leaf<TR>(a, sm, mrows, f.w, st.tau + (long long)f.k * g.n + f.j0);
 #pragma unroll
       for (int i = 0; i < TR; i++) {
         const int r = tid + BT * i;
@@ -333,7 +341,7 @@ __global__ void __launch_bounds__(BT, 1) bsof_tall_kernel(BsofGeom g, BsofState 
       if (next) {
         if (!block_wait_geq(st, st.cnt + x2, s - lo2, &sm.flag)) return;
         if (tid == 0) st.timeline[4 * s + 3] = gtimer();
-        apply_qt_mma8<true>(sC, sC + 8 * S8, a, P, ldp, f.w, C, ldc, mrows, w2, sm);
+        apply_qt_mma8<TR, true>(sC, sC + 8 * S8, a, P, ldp, f.w, C, ldc, mrows, w2, sm);
       }
       if (tid == 0) {
         __threadfence();
@@ -377,7 +385,7 @@ __global__ void __launch_bounds__(BT, 1) bsof_tall_kernel(BsofGeom g, BsofState 
     const int w2 = min(g.NB, g.n - t2 * g.NB);
     if (!block_wait_geq(st, st.cnt + x2, s - lo2, &sm.flag)) return;
     double none[TR][8];
-    apply_qt_mma8<false>(sC, sC + 8 * S8, none, P, ldp, f.w, C, ldc, mrows, w2, sm);
+    apply_qt_mma8<TR, false>(sC, sC + 8 * S8, none, P, ldp, f.w, C, ldc, mrows, w2, sm);
     if (tid == 0) {
       __threadfence();
       red_release_add(st.cnt + x2, 1);
@@ -385,23 +393,34 @@ __global__ void __launch_bounds__(BT, 1) bsof_tall_kernel(BsofGeom g, BsofState 
   }
 }
 
-constexpr size_t kTallSmem = sizeof(double) * 2 * 8 * (size_t)S8;
-}  // namespace
-
-cudaError_t launch_bsof_tall(const BsofGeom& g, const BsofState& st, int workers, cudaStream_t s) {
-  if (2 * g.n > TR * BT) return cudaErrorInvalidValue;
+template <int TR>
+cudaError_t launch_tr(const BsofGeom& g, const BsofState& st, int workers, cudaStream_t s) {
+  constexpr size_t smem = sizeof(double) * 2 * 8 * (size_t)Stage8<TR>::S8;
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(bsof_tall_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kTallSmem);
+    e = cudaFuncSetAttribute(bsof_tall_kernel<TR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem);
   if (e != cudaSuccess) return e;
   void* args[] = {(void*)&g, (void*)&st};
-  return cudaLaunchCooperativeKernel((const void*)bsof_tall_kernel, dim3(min(1 + workers, sms)),
-                                     dim3(BT), args, kTallSmem, s);
+  return cudaLaunchCooperativeKernel((const void*)bsof_tall_kernel<TR>,
+                                     dim3(min(1 + workers, sms)), dim3(BT), args, smem, s);
+}
+}  // namespace
+
+cudaError_t launch_bsof_tall(const BsofGeom& g, const BsofState& st, int workers, cudaStream_t s) {
+  if (2 * g.n <= 4 * BT) return launch_tr<4>(g, st, workers, s);
+  if (2 * g.n <= 5 * BT) return launch_tr<5>(g, st, workers, s);
+  if (2 * g.n <= 6 * BT) return launch_tr<6>(g, st, workers, s);
+  return cudaErrorInvalidValue;
 }
 
-cudaError_t preload_bsof_tall(size_t* local) { return preload_one(bsof_tall_kernel, local); }
+cudaError_t preload_bsof_tall(size_t* local) {
+  cudaError_t e;
+  if ((e = preload_one(bsof_tall_kernel<4>, local)) != cudaSuccess) return e;
+  if ((e = preload_one(bsof_tall_kernel<5>, local)) != cudaSuccess) return e;
+  return preload_one(bsof_tall_kernel<6>, local);
+}
 
 }  // namespace bsofi
