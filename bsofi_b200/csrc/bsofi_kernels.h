@@ -59,6 +59,13 @@ cudaError_t launch_bsof_persistent(double* A, long long ld, int n, int L, double
                                    int workers, cudaStream_t st, int s_begin = 0,
                                    int s_end = -1, double* Al = nullptr, long long ldl = 0);
 
+// G_k = Q_k^T of every panel from the reflectors below A's panel diagonals and
+// the compact-WY factors T of leaves of nbw columns (kernels_bsof.cu).  Only
+// where form_q_fits.
+bool form_q_fits(int n);
+cudaError_t launch_form_q(const double* A, long long ld, int n, int L, const double* T,
+                          int maxleaves, int nbw, double* G, cudaStream_t st);
+
 // Persistent BSTRI row recurrence (kernels_bstri.cu): done is (L-2) x
 // bstri_recurrence_ctmax(n, L) ints and next one int, zeroed before.
 int bstri_recurrence_ctmax(int n, int L);

@@ -1160,11 +1160,113 @@ __global__ void __launch_bounds__(K::THREADS, 1) bsof_persistent_kernel(BsofGeom
   }
 }
 
+// ------------------------------------------------------------------ Q_k^T
+// G_k = Q_k^T of every panel from the stored reflectors and the leaves' T, for
+// callers whose BSOI comes with a state of its own (reference: the dormqr of
+// lapackXbsoi_ormqr, src/bsofi_cpu.c:234-245).  A CTA owns 16 columns of one
+// G_k: they stay in its registers, from the identity on, while the panel's
+// leaves pass through shared memory, so G is written once and read never.
+// What bounds it: the FP64 tensor pipe (four m16n8k8 per 8 rows and leaf) and
+// the barriers around W; two or more CTAs an SM overlap them.  Before, one
+// launch per leaf read and wrote all of G: 653 us at n = 144, p = 20 and 445 us
+// at n = 100, p = 64 (a few tens of them products at the tensor rate); now 59 and
+// 64 us.
+struct FormQArgs {
+  const double* A;
+  long long ld;
+  int n, L;
+  const double* T;  // 256 doubles per leaf: (k * maxleaves + l) * 256
+  int maxleaves, nbw;
+  double* G;
+};
+
+template <class K, int PER>
+__global__ void __launch_bounds__(K::MT, PER) form_q_kernel(FormQArgs s) {
+  extern __shared__ __align__(16) double dyn_bsof[];
+  __shared__ __align__(16) ChainSmem<K::MW> sm;
+  constexpr int MW = K::MW, MT = K::MT, NIW = K::NIW;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int gq = lane >> 2, t = lane & 3, gc = col_of(gq);
+  const int n = s.n, n2 = 2 * n, SV = tile_stride(n), nb = (n2 + 7) / 8;
+  double* sV = dyn_bsof;
+  double* part = sV + 16 * SV;
+  // The last panel has twice the leaves: first.
+  const int k = s.L - 2 - blockIdx.y, x0 = blockIdx.x * 16;
+  const int refl = k == s.L - 2 ? n2 : n;
+  double c[NIW][2][2];
+#pragma unroll
+  for (int i = 0; i < NIW; i++)
+#pragma unroll
+    for (int cs = 0; cs < 2; cs++)
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+        c[i][cs][h] = 8 * (warp + i * MW) + 2 * t + h == x0 + gc + 8 * cs ? 1.0 : 0.0;
+  for (int j0 = 0, l = 0; j0 < refl; j0 += s.nbw, l++) {
+    const int w = min(s.nbw, refl - j0);
+    const double* P = s.A + cm((long long)k * n, (long long)k * n + j0, s.ld);  // row 0
+    const bool vec = pair_aligned(P, s.ld);
+    const double* T = s.T + ((long long)k * s.maxleaves + l) * 256;
+    // Rows from j0 + 16 on as stored, the 16 above masked to unit lower
+    // trapezoidal; zero up to a full block and in columns beyond the leaf.
+    for (int cc = warp; cc < 16; cc += MW) {
+      const double* col = P + cm(0, cc, s.ld);
+      if (cc < w && vec) {
+        for (int r = j0 + 16 + 2 * lane; r < 8 * nb; r += 64)
+          cp_async16(sV + sidx(r, cc, SV), r < n2 ? col + r : col, r + 1 < n2 ? 16 : (r < n2 ? 8 : 0));
+      } else {
+        for (int r = j0 + 16 + lane; r < 8 * nb; r += 32)
+          sV[sidx(r, cc, SV)] = cc < w && r < n2 ? col[r] : 0.0;
+      }
+    }
+    cp_async_commit();
+    for (int e = tid; e < 256; e += MT) {
+      const int r = e & 15, cc = e >> 4;
+      double v = 0.0;
+      if (cc < w && j0 + r < n2) v = r == cc ? 1.0 : (r > cc ? P[cm(j0 + r, cc, s.ld)] : 0.0);
+      if (j0 + r < 8 * nb) sV[sidx(j0 + r, cc, SV)] = v;
+      sm.T[r][cc] = T[e];
+    }
+    cp_async_wait<0>();
+    bar_main<MT>();
+    double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+#pragma unroll
+    for (int i = 0; i < NIW; i++) {
+      const int b = warp + i * MW;
+      if (8 * b + 7 >= j0 && b < nb) {
+#pragma unroll
+        for (int jt = 0; jt < 2; jt++) {
+          const double2 v =
+              *reinterpret_cast<const double2*>(sV + sidx(8 * b + 2 * t, gc + 8 * jt, SV));
+          dmma_16x8x8(acc[jt], c[i][0][0], c[i][1][0], c[i][0][1], c[i][1][1], v.x, v.y);
+        }
+      }
+    }
+    double fr[2][4];
+    reduce_w<MW>(acc, fr, part, sm, gq, t, warp);
+#pragma unroll
+    for (int i = 0; i < NIW; i++) {
+      const int b = warp + i * MW;
+      if (8 * b + 7 >= j0 && b < nb) update_block(c[i], fr, sV, SV, 8 * b, gq, t);
+    }
+    bar_main<MT>();  // V, T and W are no longer read
+  }
+  double* C = s.G + (long long)k * n2 * n2 + cm(0, x0, n2);
+#pragma unroll
+  for (int i = 0; i < NIW; i++) {
+    const int b = warp + i * MW;
+#pragma unroll
+    for (int cs = 0; cs < 2; cs++)
+      st_pair(C + cm(0, gc + 8 * cs, n2), 8 * b + 2 * t, n2, b < nb && x0 + gc + 8 * cs < n2, true,
+              c[i][cs][0], c[i][cs][1]);
+  }
+}
+
 // ------------------------------------------------------------------ launcher
 using Chain64 = ChainCfg<3, 5, 4>;
 using Chain128 = ChainCfg<7, 5, 4>;
 using Chain256 = ChainCfg<7, 9, 8>;
 using Chain400 = ChainCfg<7, 14, 13>;
+using Chain640 = ChainCfg<7, 23, 20>;  // (its worker shape only: form_q_kernel)
 
 // 16-wide leaves up to n = 400, where the next tile still fits in shared
 // memory beside V; the tall kernel's 8-wide ones above.
@@ -1239,12 +1341,47 @@ cudaError_t launch_bsof_persistent(double* A, long long ld, int n, int L, double
   return launch_bsof_tall(g, s, workers, st);
 }
 
+template <class K, int PER>
+static cudaError_t launch_form_q_cfg(const FormQArgs& a, cudaStream_t st) {
+  static PerDevice once;
+  const int dev = once.pending();
+  if (dev >= 0) {
+    const size_t most =
+        sizeof(double) * (16 * (size_t)tile_stride(K::MAX_ROWS / 2) + 256 * K::MW);
+    cudaError_t e = cudaFuncSetAttribute(form_q_kernel<K, PER>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (e != cudaSuccess) return e;
+    once.mark(dev);
+  }
+  form_q_kernel<K, PER><<<dim3((2 * a.n + 15) / 16, a.L - 1), K::MT,
+                          sizeof(double) * (16 * (size_t)tile_stride(a.n) + 256 * K::MW), st>>>(a);
+  return cudaGetLastError();
+}
+
+bool form_q_fits(int n) { return 2 * n <= Chain640::MAX_ROWS; }
+
+cudaError_t launch_form_q(const double* A, long long ld, int n, int L, const double* T,
+                          int maxleaves, int nbw, double* G, cudaStream_t st) {
+  const FormQArgs a = {A, ld, n, L, T, maxleaves, nbw, G};
+  if (2 * n <= Chain64::MAX_ROWS) return launch_form_q_cfg<Chain64, 4>(a, st);
+  if (2 * n <= Chain128::MAX_ROWS) return launch_form_q_cfg<Chain128, 2>(a, st);
+  if (2 * n <= Chain256::MAX_ROWS) return launch_form_q_cfg<Chain256, 2>(a, st);
+  if (2 * n <= Chain400::MAX_ROWS) return launch_form_q_cfg<Chain400, 1>(a, st);
+  if (2 * n <= Chain640::MAX_ROWS) return launch_form_q_cfg<Chain640, 1>(a, st);
+  return cudaErrorInvalidValue;
+}
+
 cudaError_t preload_bsof(size_t* local) {
   cudaError_t e;
   if ((e = preload_one(bsof_persistent_kernel<Chain64>, local)) != cudaSuccess) return e;
   if ((e = preload_one(bsof_persistent_kernel<Chain128>, local)) != cudaSuccess) return e;
   if ((e = preload_one(bsof_persistent_kernel<Chain256>, local)) != cudaSuccess) return e;
   if ((e = preload_one(bsof_persistent_kernel<Chain400>, local)) != cudaSuccess) return e;
+  if ((e = preload_one(form_q_kernel<Chain64, 4>, local)) != cudaSuccess) return e;
+  if ((e = preload_one(form_q_kernel<Chain128, 2>, local)) != cudaSuccess) return e;
+  if ((e = preload_one(form_q_kernel<Chain256, 2>, local)) != cudaSuccess) return e;
+  if ((e = preload_one(form_q_kernel<Chain400, 1>, local)) != cudaSuccess) return e;
+  if ((e = preload_one(form_q_kernel<Chain640, 1>, local)) != cudaSuccess) return e;
   return preload_bsof_tall(local);
 }
 

@@ -741,7 +741,8 @@ int run_bsoftri(int n, int L, double* dA, int ldd, double* dtau, void* ws, cudaS
 }
 
 // G_k = Q_k^T of every panel from the stored reflectors and tau: compact-WY
-// factors first, then the block reflectors applied to identity matrices.
+// factors first, then the block reflectors applied to identity matrices (one
+// launch for all leaves; above the limit of its registers one per leaf).
 int bsoi_form_q(int n, int L, double* dA, int ldd, const double* dtau, void* ws, cudaStream_t st) {
   Layout ly = layout(n, L, ldd);
   double* Tb = at<double>(ws, ly.T);
@@ -751,6 +752,10 @@ int bsoi_form_q(int n, int L, double* dA, int ldd, const double* dtau, void* ws,
   build_leaf_t_kernel<<<dim3(ly.maxleaves, L - 1), 256, 0, st>>>(dA, ldd, n, L, dtau, Tb,
                                                                   ly.maxleaves, ly.nbw);
   CK(cudaGetLastError());
+  if (form_q_fits(n)) {
+    CK(launch_form_q(dA, ldd, n, L, Tb, ly.maxleaves, ly.nbw, G, st));
+    return 0;
+  }
   CK(launch_set_identity(G, n2, n2, g2, L - 1, st));
   for (int l = 0, j0 = 0; j0 < n2; l++, j0 += ly.nbw) {
     // Regular panels k = 0..L-3 have n reflectors, the last one 2n.
