@@ -69,6 +69,9 @@ struct ChainCfg {
   static constexpr int HW = 4;  // helper warps: one builds T, the others load and store
   static constexpr int THREADS = MT + 32 * HW;
   static constexpr int CT = MT + 32;  // column barrier: with the T warp, the last helper
+  // Largest panel height 2n: rows owned by the chain's warps and a worker's.
+  static constexpr int ROWS_CHAIN = 8 * (2 + FW * NI), ROWS_WORK = 8 * MW * NIW;
+  static constexpr int MAX_ROWS = ROWS_CHAIN < ROWS_WORK ? ROWS_CHAIN : ROWS_WORK;
   // Row slots are taken in groups of GS, skipped when every row is finished.
   static constexpr int GS = 3, NG = (NI + GS - 1) / GS;
   // Tiles move between global and shared memory by bulk copies, which keep the
@@ -76,6 +79,8 @@ struct ChainCfg {
   // chain waits for the workers' answer and latency counts) by cp.async and
   // by stores of the warps that hold the reflectors.
   static constexpr bool BULK = NI > 5;
+  // Loads a lane and column in flight where columns are copied by plain loads.
+  static constexpr int LOADS = ROWS_WORK <= 128 ? 4 : (ROWS_WORK <= 256 ? 8 : 16);
   // V as the operand of W = V^T C comes from the registers that factored it,
   // or, where V and C do not fit in registers together, from shared memory.
   static constexpr bool VREG = NI <= 9;
@@ -83,9 +88,6 @@ struct ChainCfg {
   // gives most of its own to the two that compute
   // (2 x 128 x 224 + 128 x 56 = 384 x 168).
   static constexpr bool REGS = THREADS == 384;
-  // Largest panel height 2n: rows owned by the chain's warps and a worker's.
-  static constexpr int ROWS_CHAIN = 8 * (2 + FW * NI), ROWS_WORK = 8 * MW * NIW;
-  static constexpr int MAX_ROWS = ROWS_CHAIN < ROWS_WORK ? ROWS_CHAIN : ROWS_WORK;
   static_assert(MW == 4 || MW == 8, "partial sums are read as 4 or 8 per column");
 };
 
@@ -250,6 +252,32 @@ BSOFI_DEVINL void st_pair(double* col, int r, int rows, bool ok, bool vec, doubl
   } else {
     if (r < rows) __stcg(col + r, x);
     if (r + 1 < rows) __stcg(col + r + 1, y);
+  }
+}
+// Rows [r0, r1) of NC columns (c, c + step, .., those below c1) of a tile that
+// breaks 16-byte alignment, from src (leading dimension ld) to dst (column
+// stride S) by one warp, U loads a lane and column in flight (through L2:
+// cp.async of 8 bytes would leave lines in this SM's L1 that other SMs still
+// write).
+template <int NC, int U>
+BSOFI_DEVINL void copy_cols(double* dst, int S, const double* src, long long ld, int c, int step,
+                            int c1, int r0, int r1, int lane) {
+  for (int r = r0 + lane; r < r1; r += 32 * U) {
+    double v[NC][U];
+#pragma unroll
+    for (int j = 0; j < NC; j++) {
+      const double* p = src + cm(r, c + j * step, ld);
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        v[j][u] = c + j * step < c1 && r + 32 * u < r1 ? __ldcg(p + 32 * u) : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < NC; j++) {
+      double* q = dst + (c + j * step) * S + r;
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (c + j * step < c1 && r + 32 * u < r1) q[32 * u] = v[j][u];
+    }
   }
 }
 BSOFI_DEVINL bool pair_aligned(const double* p, long long ld) {
@@ -694,6 +722,18 @@ BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const dou
             }
           }
         }
+        if (!vec) {
+          constexpr int NC = 16 / K::LOADS;
+#pragma unroll 1
+          for (int c = hw; c < z.w2; c += NC * LW) {
+            copy_cols<NC, K::LOADS>(sC, SC, z.C, z.ldc, c, LW, z.w2, z.ab, z.rows, lane);
+            if (z.fresh) {
+              const double* F = z.C + 2 * n;
+              copy_cols<NC, K::LOADS>(sC + f0, SC, F, z.ldc, c, LW, z.w2, 0, q0, lane);
+              copy_cols<NC, K::LOADS>(sC - q0, SC, F, z.ldc, c, LW, z.w2, q0, n, lane);
+            }
+          }
+        }
 #pragma unroll 1
         for (int c = hw; c < 16; c += LW) {
           const double* col = z.C + cm(0, c, z.ldc);
@@ -709,14 +749,6 @@ BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const dou
 #pragma unroll 1
               for (int q = 2 * lane; q < n; q += 64)
                 cp_async16(sC + sidx(q < q0 ? f0 + q : q - q0, c, SC), col + 2 * n + q, 16);
-            }
-          } else if (!vec) {
-#pragma unroll 4
-            for (int r = z.ab + lane; r < z.rows; r += 32) sC[sidx(r, c, SC)] = __ldcg(col + r);
-            if (z.fresh) {
-#pragma unroll 4
-              for (int q = lane; q < n; q += 32)
-                sC[sidx(q < q0 ? f0 + q : q - q0, c, SC)] = __ldcg(col + 2 * n + q);
             }
           }
           // Zero rows up to a full block.
@@ -1066,6 +1098,11 @@ BSOFI_DEVINL void worker(const BsofGeom& g, const BsofState& st, double* sV, dou
         for (int cc = 0; cc < f.w; cc++)
           bulk_load(sV + sidx(16, cc, SV), P + cm(16, cc, ldp), rows - 16, &sm.bar);
       }
+      if (!vec) {
+#pragma unroll
+        for (int cc = warp; cc < 16; cc += 2 * MW)
+          copy_cols<2, K::LOADS>(sV, SV, P, ldp, cc, MW, f.w, 16, rows, lane);
+      }
       for (int cc = warp; cc < 16; cc += MW) {
         const double* col = P + cm(0, cc, ldp);
         if (cc >= f.w) {
@@ -1077,10 +1114,8 @@ BSOFI_DEVINL void worker(const BsofGeom& g, const BsofState& st, double* sV, dou
               cp_async16(sV + sidx(r, cc, SV), col + r, 16);
           }
           if (lane < 8 && max(rows, 16) + lane < 8 * nb) sV[sidx(max(rows, 16) + lane, cc, SV)] = 0.0;
-        } else {
-#pragma unroll 8
-          for (int r = 16 + lane; r < 8 * nb; r += 32)
-            sV[sidx(r, cc, SV)] = r < rows ? __ldcg(col + r) : 0.0;
+        } else if (lane < 8 && max(rows, 16) + lane < 8 * nb) {
+          sV[sidx(max(rows, 16) + lane, cc, SV)] = 0.0;
         }
       }
       const double* T = st.T + ((long long)f.k * st.maxleaves + f.l) * 256;
