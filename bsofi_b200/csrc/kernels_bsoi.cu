@@ -611,9 +611,11 @@ cudaError_t launch_bsoi_persistent(double* A, long long ld, double* carry0, doub
   // Row range in rows here; launch_al turns it into row bands of its tiles.
   s.rb0 = row0;
   s.rb1 = row1 < 0 ? s.N : row1;
+  // (16-byte copies take row pairs of the matrix and the carries and pairs of
+  // K inside a column of G, whose leading dimension is 2n: n may be odd.)
   const bool al = ((uintptr_t)A % 16 == 0) && ((uintptr_t)carry0 % 16 == 0) &&
                   ((uintptr_t)carry1 % 16 == 0) && ((uintptr_t)G % 16 == 0) && ld % 2 == 0 &&
-                  ldc % 2 == 0 && n % 2 == 0;
+                  ldc % 2 == 0;
   if (gemm_k16()) {
     if (small) return al ? launch_al<CfgS16, true>(s, st) : launch_al<CfgS16, false>(s, st);
     return al ? launch_al<CfgM16, true>(s, st) : launch_al<CfgM16, false>(s, st);

@@ -51,10 +51,11 @@ template <class Cfg>
 static cudaError_t run(const GemmDims& d, const GemmA& a, const GemmB& b, const GemmC& c,
                        int batch, cudaStream_t st) {
   dim3 grid((d.M + Cfg::BM - 1) / Cfg::BM, (d.N + Cfg::BN - 1) / Cfg::BN, batch);
+  // 16-byte copies take row pairs of A and, in B, pairs of K inside a column:
+  // where A's K segments split does not matter.
   bool aligned = al16(a.p0) && (a.p1 == nullptr || al16(a.p1)) && al16(b.p) &&
                  (a.ld0 % 2 == 0) && (a.ld1 % 2 == 0) && (b.ld % 2 == 0) &&
-                 (a.bs0 % 2 == 0) && (a.bs1 % 2 == 0) && (b.bs % 2 == 0) &&
-                 (a.ksplit % 2 == 0);
+                 (a.bs0 % 2 == 0) && (a.bs1 % 2 == 0) && (b.bs % 2 == 0);
   if (aligned)
     gemm_kernel<Cfg, true><<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(d, a, b, c);
   else

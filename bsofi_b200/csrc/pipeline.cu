@@ -1233,8 +1233,7 @@ int bsofi_dev_bsoi_group_run(int count, const int* n, const int* L, double* cons
       I.tile0 = G.total;
       G.total += bsoi_group_tiles(n[i], L[i], g == 0);
       al = al && ((uintptr_t)I.A % 16 == 0) && ((uintptr_t)I.carry[0] % 16 == 0) &&
-           ((uintptr_t)I.carry[1] % 16 == 0) && ((uintptr_t)I.G % 16 == 0) && I.ld % 2 == 0 &&
-           I.n % 2 == 0;
+           ((uintptr_t)I.carry[1] % 16 == 0) && ((uintptr_t)I.G % 16 == 0) && I.ld % 2 == 0;
     }
   }
   return 0;
