@@ -123,22 +123,30 @@ void bsofi_device_set_batch_chains(int k) {
 static int g_pipelined = 1;
 void bsofi_device_set_batch_pipelined(int on) { flag_set(&g_pipelined, on ? 1 : 0); }
 
-/* BSOF worker CTAs per instance of a batch (0: by block size).  Measured on
- * pipelined batches: 16 x (n = 256, p = 32) ran 134 inversions/s with 6
- * workers and 142 with 12; the 256 instances of mixed sizes (n = 64..256)
- * ran 268.5/s with 6 for all, 253/s with 12 for all, 251/s with 3.  So the
- * largest 16-wide instances take 12, smaller ones 6, 8-wide ones 24. */
+/* BSOF worker CTAs per instance of a batch (0: by block size and the number of
+ * instances in flight).  A chain's workers hold their SMs while it runs, so
+ * the best count falls as more chains run together; with few chains the large
+ * blocks end last and take more.  Measured on pipelined batches of mixed sizes
+ * (n = 64..256, p = 8..64; ms a batch with 6 workers below n = 224 and 12 from
+ * there on -> with this rule): 48 instances 230.6 -> 223.7, 20 90.5 -> 87.3,
+ * 16 67.9 -> 67.2, 14 96.8 -> 94.4, 12 40.9 -> 41.2 and 32.3 -> 31.2, 9
+ * 48.6 -> 34.6, 7 30.0 -> 18.5, 4 44.0 -> 32.4.  The line at 12 in flight: 13 and
+ * 16 instances took 79.8 and 67.1 with 10 for all, 85.1 and 70.6 with 14 and 12
+ * for the large ones; 12 instances 36.8 with 10 for all, 31.2 with 16 and 8.
+ * Panels of n > 256 take 24. */
 static int g_batch_workers = 0;
 void bsofi_device_set_batch_workers(int w) { flag_set(&g_batch_workers, w < 0 ? 0 : w); }
-static int batch_workers(int n) {
+static int batch_workers(int n, int in_flight) {
   const int w = flag_get(&g_batch_workers);
   if (w > 0) return w;
-  return n > 256 ? 24 : (n >= 224 ? 12 : 6);
+  if (n > 256) return 24;
+  if (in_flight > 12) return 10;
+  return n >= 180 || in_flight < 6 ? 16 : 96 / in_flight;
 }
 
 /* The same settings for the server's requests (server.c). */
 int bsofi_batch_pipelined_now(void) { return flag_get(&g_pipelined); }
-int bsofi_batch_workers_for(int n) { return batch_workers(n); }
+int bsofi_batch_workers_for(int n) { return batch_workers(n, MAX_STREAMS); }
 
 unsigned long long bsofi_batch_workspace_bytes_ex(int count, const int *n, const int *L,
                                                   const int *ldda, int precision) {
@@ -198,7 +206,7 @@ static int grouped_fp64(stream_pool *p, int used, int count, const int *n, const
   }
   for (i = 0; i < count && !r; i++) {
     const int k = ord[i].i;
-    const int workers = batch_workers(n[k]);
+    const int workers = batch_workers(n[k], used);
     r = bsofi_dev_bsoftri_q_ex(n[k], L[k], dA[k], ldda[k], dtau[k], ws[k], p->s[i % used],
                                workers);
     *launches += bsofi_dev_launch_count();
@@ -288,7 +296,7 @@ int bsofi_device_invert_batched_ex(int count, const int *n, const int *L, double
     bsofi_dev_set_nonpersistent(1);
     for (i = 0; i < count && !r; i++) {
       const int k = ord[i].i, slot = i % used;
-      const int workers = batch_workers(n[k]);
+      const int workers = batch_workers(n[k], used);
       r = bsofi_dev_invert_two_streams(n[k], L[k], dA[k], ldda[k], dtau[k],
                                        (char *)dwork + off[k], p->hi[slot], p->s[slot],
                                        p->gate[slot], workers,
@@ -304,7 +312,7 @@ int bsofi_device_invert_batched_ex(int count, const int *n, const int *L, double
   for (i = 0; i < count && !(precision == 0 && grouped) && !pipelined; i++) {
     const int k = ord[i].i;
     /* Few BSOF workers per instance: the batch supplies the parallelism. */
-    const int workers = batch_workers(n[k]);
+    const int workers = batch_workers(n[k], used);
     /* Gate: instance i waits for the chain of instance i - K (ring slot
      * i % K, recorded by that instance after its BSOF) and records the slot
      * after its own; the host issues them in that order. */
