@@ -210,7 +210,7 @@ BSOFI_DEVINL bool block_wait_geq(const BsofState& st, const int* p, int target, 
   return ok;
 }
 
-// n above the 16-wide leaves' limit (kernels_bsof_tall.cu).
+// n above kernels_bsof.cu's limit (kernels_bsof_tall.cu).
 cudaError_t launch_bsof_tall(const BsofGeom& g, const BsofState& st, int workers, cudaStream_t s);
 cudaError_t preload_bsof_tall(size_t* local);
 

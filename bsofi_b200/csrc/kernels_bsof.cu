@@ -62,15 +62,16 @@ namespace bsofi {
 // FW row warps of NI 8-row blocks each, one top warp, helper warps (which
 // stage the next tile in shared memory beside V while the leaf is factored).
 // NIW: 8-row blocks per warp of a worker (all FW + 1 warps take rows there).
-template <int FW_, int NI_, int NIW_>
+// CN: columns per lane; leaves and tiles are LW = 8 CN wide.
+template <int FW_, int NI_, int NIW_, int CN_ = 2>
 struct ChainCfg {
-  static constexpr int FW = FW_, NI = NI_, NIW = NIW_;
+  static constexpr int FW = FW_, NI = NI_, NIW = NIW_, CN = CN_, LW = 8 * CN;
   static constexpr int MW = FW + 1, MT = 32 * MW;
   static constexpr int HW = 4;  // helper warps: one builds T, the others load and store
   static constexpr int THREADS = MT + 32 * HW;
   static constexpr int CT = MT + 32;  // column barrier: with the T warp, the last helper
   // Largest panel height 2n: rows owned by the chain's warps and a worker's.
-  static constexpr int ROWS_CHAIN = 8 * (2 + FW * NI), ROWS_WORK = 8 * MW * NIW;
+  static constexpr int ROWS_CHAIN = 8 * (CN + FW * NI), ROWS_WORK = 8 * MW * NIW;
   static constexpr int MAX_ROWS = ROWS_CHAIN < ROWS_WORK ? ROWS_CHAIN : ROWS_WORK;
   // Row slots are taken in groups of GS, skipped when every row is finished.
   static constexpr int GS = 3, NG = (NI + GS - 1) / GS;
@@ -79,11 +80,18 @@ struct ChainCfg {
   // chain waits for the workers' answer and latency counts) by cp.async and
   // by stores of the warps that hold the reflectors.
   static constexpr bool BULK = NI > 5;
-  // Loads a lane and column in flight where columns are copied by plain loads.
+  // Loads a lane and column in flight where unaligned columns are copied by plain loads
+  // (16-wide forms: their chain does not wait for them; the 8-wide ones use spans).
   static constexpr int LOADS = ROWS_WORK <= 128 ? 4 : (ROWS_WORK <= 256 ? 8 : 16);
   // V as the operand of W = V^T C comes from the registers that factored it,
   // or, where V and C do not fit in registers together, from shared memory.
-  static constexpr bool VREG = NI <= 9;
+  static constexpr bool VREG = NI * CN <= 23;
+  // EARLY: a leaf is published when V is in shared memory, not when the next tile
+  // is, so that the workers' answer may take a chain step longer.  Where the chain
+  // waits for them, an inversion at n = 576, p = 12 went from 19.6 to 17.6 ms and at
+  // n = 529 from 20.3 to 18.0; up to n = 400 it does not wait, and the extra barrier
+  // costs (n = 256, p = 32 11.65 -> 11.82, n = 400, p = 16 12.9 -> 13.3).
+  static constexpr bool EARLY = CN == 1;
   // With 12 warps a thread gets 168 registers at launch; the helper warpgroup
   // gives most of its own to the two that compute
   // (2 x 128 x 224 + 128 x 56 = 384 x 168).
@@ -93,8 +101,8 @@ struct ChainCfg {
 
 // Leaf s as the chain CTA sees it.  Rows are counted from the top of the
 // panel, except in the second half of the final panel when n is not a
-// multiple of 16: there from its row n on, so that a leaf's first row is
-// always a multiple of 16.
+// multiple of the leaf width: there from its row n on, so that a leaf's first
+// row is always a multiple of it.
 struct ChainStep {
   Leaf f;
   int base, ab, rows, nb;  // first row counted, the leaf's first row, panel rows, 8-row blocks
@@ -105,7 +113,7 @@ struct ChainStep {
 };
 
 BSOFI_DEVINL int leaf_base(const BsofGeom& g, const Leaf& f) {
-  return (f.k == g.L - 2 && f.l >= g.nl && (g.n & 15) != 0) ? g.n : 0;
+  return (f.k == g.L - 2 && f.l >= g.nl && g.n % g.NB != 0) ? g.n : 0;
 }
 
 BSOFI_DEVINL ChainStep chain_step(const BsofGeom& g, const BsofState& st, int s) {
@@ -125,12 +133,12 @@ BSOFI_DEVINL ChainStep chain_step(const BsofGeom& g, const BsofState& st, int s)
     tile_range(g, c.m2, c.t2, c.lo2, hi2);
     c.C = tile_ptr(g, st, c.f.k, c.base, c.m2, c.t2, c.ldc);
   }
-  c.P = mat_ptr(g, st, (long long)c.f.k * g.n + c.base, c.f.m, c.f.t * 16, c.ldp);
-  c.w2 = min(16, g.n - c.t2 * 16);
+  c.P = mat_ptr(g, st, (long long)c.f.k * g.n + c.base, c.f.m, c.f.t * g.NB, c.ldp);
+  c.w2 = min(g.NB, g.n - c.t2 * g.NB);
   // Panel change (rows shift by n, n fresh rows come in), and the shift by n
-  // inside the final panel when n is not a multiple of 16.
+  // inside the final panel when n is not a multiple of the leaf width.
   c.fresh = c.next && c.f.l == g.nl - 1 && c.f.k <= g.L - 3;
-  c.trans = c.fresh || (c.next && c.f.l == g.nl - 1 && (g.n & 15) != 0);
+  c.trans = c.fresh || (c.next && c.f.l == g.nl - 1 && g.n % g.NB != 0);
   return c;
 }
 
@@ -150,6 +158,7 @@ struct ChainSmem {
   };
   ChainStep step[2];       // of leaves s, s+1
   uint64_t bar;            // bulk loads
+  int ok[2];               // the next tile of an even / odd leaf arrived
   int flag;
   int task;
 };
@@ -205,9 +214,28 @@ template <int COUNT>
 BSOFI_DEVINL void bar_col() {
   asm volatile("bar.sync 4, %0;" ::"n"(COUNT) : "memory");
 }
+// Per leaf: V, T and the next tile are in shared memory (the T warp only
+// arrives); the leaf is done.
 template <int COUNT>
-BSOFI_DEVINL void bar_all() {
+BSOFI_DEVINL void bar_ready() {
   asm volatile("bar.sync 3, %0;" ::"n"(COUNT) : "memory");
+}
+template <int COUNT>
+BSOFI_DEVINL void bar_ready_arrive() {
+  asm volatile("bar.arrive 3, %0;" ::"n"(COUNT) : "memory");
+}
+template <int COUNT>
+BSOFI_DEVINL void bar_done() {
+  asm volatile("bar.sync 6, %0;" ::"n"(COUNT) : "memory");
+}
+// V is in shared memory: the factoring warps arrive, the T warp waits.
+template <int COUNT>
+BSOFI_DEVINL void bar_v() {
+  asm volatile("bar.sync 5, %0;" ::"n"(COUNT) : "memory");
+}
+template <int COUNT>
+BSOFI_DEVINL void bar_v_arrive() {
+  asm volatile("bar.arrive 5, %0;" ::"n"(COUNT) : "memory");
 }
 template <int COUNT>
 BSOFI_DEVINL void bar_help() {
@@ -282,6 +310,58 @@ BSOFI_DEVINL void copy_cols(double* dst, int S, const double* src, long long ld,
 }
 BSOFI_DEVINL bool pair_aligned(const double* p, long long ld) {
   return ((reinterpret_cast<uintptr_t>(p) & 15) == 0) && ((ld & 1) == 0);
+}
+
+// cnt elements of one column from src (8-byte aligned) to dst (16-byte aligned)
+// with bulk copies, which need 16 bytes on both sides: from an odd address the
+// copy starts at the second element and lands one element late (never beyond
+// dst[cnt - 1]); once it has arrived a warp moves it down and fetches the edges.
+BSOFI_DEVINL int span_late(const double* src) {
+  return (int)(reinterpret_cast<uintptr_t>(src) >> 3) & 1;
+}
+BSOFI_DEVINL int span_bulk(const double* src, int cnt) {
+  return max(0, cnt - 2 * span_late(src)) & ~1;
+}
+BSOFI_DEVINL void span_issue(double* dst, const double* src, int cnt, uint64_t* bar) {
+  const int late = span_late(src), m = span_bulk(src, cnt);
+  if (m > 0) bulk_load(dst + 2 * late, src + late, m, bar);
+}
+BSOFI_DEVINL void span_finish(double* dst, const double* src, int cnt, int lane) {
+  const int late = span_late(src), m = span_bulk(src, cnt);
+  const int edge = late && lane == 0 ? 0 : m + lane;  // the first element, and those past the copy
+  const bool mine = lane < 3 && edge < cnt;
+  const double v = mine ? __ldcg(src + edge) : 0.0;
+  if (late) {
+    constexpr int U = 8;
+#pragma unroll 1
+    for (int r = 1 + lane; r - lane <= m; r += 32 * U) {
+      double x[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) x[u] = r + 32 * u <= m ? dst[r + 32 * u + 1] : 0.0;
+      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (r + 32 * u <= m) dst[r + 32 * u] = x[u];
+      __syncwarp();
+    }
+  }
+  if (mine) dst[edge] = v;
+}
+
+// One thread's start of all w columns (vec: none of them needs span_finish).
+BSOFI_DEVINL void issue_columns(double* dst, int S, const double* src, long long ld, int w, int cnt,
+                                bool vec, uint64_t* bar) {
+  int total = w * cnt;
+  if (!vec) {
+    total = 0;
+    for (int c = 0; c < w; c++) total += span_bulk(src + cm(0, c, ld), cnt);
+  }
+  fence_proxy();
+  tc::mbar_arrive_expect_tx(bar, 8 * total);
+  for (int c = 0; c < w; c++) {
+    if (vec) bulk_load(dst + c * S, src + cm(0, c, ld), cnt, bar);
+    else span_issue(dst + c * S, src + cm(0, c, ld), cnt, bar);
+  }
 }
 
 // ------------------------------------------------------------ column steps
@@ -360,237 +440,254 @@ BSOFI_DEVINL double col_total(const double* red, int c, int t) {
   }
 }
 
-// Warp sums of the two columns' partial dot products into red[column][warp]:
+// Warp sums of the lane's columns' partial dot products into red[column][warp]:
 // again DMMAs with ones, whose results lane 4 g + t holds for columns 2t, 2t+1.
-template <int MW>
-BSOFI_DEVINL void put_partials(double* red, double d0, double d1, int g, int t, int warp) {
-  double e0[2] = {0.0, 0.0}, e1[2] = {0.0, 0.0};
-  dmma_8x8x4(e0, 1.0, d0);
-  dmma_8x8x4(e1, 1.0, d1);
-  if (g < 2) {
-    double* dst = red + (8 * g + 2 * t) * MW + warp;
-    dst[0] = g == 0 ? e0[0] : e1[0];
-    dst[MW] = g == 0 ? e0[1] : e1[1];
+template <class K>
+BSOFI_DEVINL void put_partials(double* red, const double (&d)[K::CN], int g, int t, int warp) {
+  double e[K::CN][2];
+#pragma unroll
+  for (int cs = 0; cs < K::CN; cs++) {
+    e[cs][0] = e[cs][1] = 0.0;
+    dmma_8x8x4(e[cs], 1.0, d[cs]);
+  }
+  if (g < K::CN) {
+    double* dst = red + (8 * g + 2 * t) * K::MW + warp;
+    dst[0] = g == 0 ? e[0][0] : e[K::CN - 1][0];
+    dst[K::MW] = g == 0 ? e[0][1] : e[K::CN - 1][1];
   }
 }
 
 // One pass of a row warp over its rows: the update by the finished pivot
-// column I (half CSU; factors f0, f1 for columns g, g+8, zero where a column
-// is finished; UPD0: some of columns g are pending) and the dot products with
-// the next pivot column J = I+1 (half CSD).  ab8: first 8-row block of the
-// leaf; nb: row blocks of the panel.
-template <class K, bool UPD0, int CSU, int CSD>
-BSOFI_DEVINL void row_pass(double (&a)[K::NI][2][2], double (&x)[K::NI][2],
-                           double f0, double f1, int srcd, int ab8, int nb, int warp,
-                           double& d0, double& d1) {
-  double s0[2] = {0.0, 0.0}, s1[2] = {0.0, 0.0};
+// column (f: factors of the lane's columns, zero where a column is finished;
+// column sets below CSU are all finished) and the dot products with the next
+// pivot column (set CSD, lane srcd).  ab8: first 8-row block of the leaf; nb:
+// row blocks of the panel.
+template <class K, int CSU, int CSD>
+BSOFI_DEVINL void row_pass(double (&a)[K::NI][K::CN][2], double (&x)[K::NI][2],
+                           const double (&f)[K::CN], int srcd, int ab8, int nb, int warp,
+                           double (&d)[K::CN]) {
+  double s[K::CN][2] = {};
 #pragma unroll
   for (int q = 0; q < K::NG; q++) {
     constexpr int GS = K::GS;
     const int ia = q * GS, ie = (ia + GS < K::NI ? ia + GS : K::NI);
-    if ((ie - 1) * K::FW + warp < ab8 || 2 + ia * K::FW + warp >= nb) continue;
+    if ((ie - 1) * K::FW + warp < ab8 || K::CN + ia * K::FW + warp >= nb) continue;
 #pragma unroll
     for (int i = ia; i < ie; i++) {
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const double xo = x[i][h];
-        if (UPD0) a[i][0][h] = fma(-xo, f0, a[i][0][h]);
-        a[i][1][h] = fma(-xo, f1, a[i][1][h]);
+#pragma unroll
+        for (int cs = CSU; cs < K::CN; cs++) a[i][cs][h] = fma(-xo, f[cs], a[i][cs][h]);
         const double xn = shfl_d(a[i][CSD][h], srcd);
         x[i][h] = xn;
-        s0[h] = fma(xn, a[i][0][h], s0[h]);
-        s1[h] = fma(xn, a[i][1][h], s1[h]);
+#pragma unroll
+        for (int cs = 0; cs < K::CN; cs++) s[cs][h] = fma(xn, a[i][cs][h], s[cs][h]);
       }
     }
   }
-  d0 = s0[0] + s0[1];
-  d1 = s1[0] + s1[1];
+#pragma unroll
+  for (int cs = 0; cs < K::CN; cs++) d[cs] = s[cs][0] + s[cs][1];
 }
 
 // The dot products with column 0, before the first column step.
 template <class K>
-BSOFI_DEVINL void row_first(double (&a)[K::NI][2][2], double (&x)[K::NI][2], int t,
-                            double& d0, double& d1) {
-  double s0[2] = {0.0, 0.0}, s1[2] = {0.0, 0.0};
+BSOFI_DEVINL void row_first(double (&a)[K::NI][K::CN][2], double (&x)[K::NI][2], int t,
+                            double (&d)[K::CN]) {
+  double s[K::CN][2] = {};
 #pragma unroll
   for (int i = 0; i < K::NI; i++)
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       const double xn = shfl_d(a[i][0][h], t);
       x[i][h] = xn;
-      s0[h] = fma(xn, a[i][0][h], s0[h]);
-      s1[h] = fma(xn, a[i][1][h], s1[h]);
+#pragma unroll
+      for (int cs = 0; cs < K::CN; cs++) s[cs][h] = fma(xn, a[i][cs][h], s[cs][h]);
     }
-  d0 = s0[0] + s0[1];
-  d1 = s1[0] + s1[1];
+#pragma unroll
+  for (int cs = 0; cs < K::CN; cs++) d[cs] = s[cs][0] + s[cs][1];
 }
 
 // Sums, reflector and v_I^T a_c of this lane's columns at column step I.
+template <class K>
 struct ColStep {
   Refl rf;
-  double w0, w1;
+  double w[K::CN];
 };
-template <int MW>
-BSOFI_DEVINL ColStep col_step(const ChainSmem<MW>& sm, int I, int g, int t) {
+template <class K>
+BSOFI_DEVINL ColStep<K> col_step(const ChainSmem<K::MW>& sm, int I, int g, int t) {
   const int buf = I & 1, ri = group_of(I & 7) + (I & 8);
-  ColStep c;
-  const double alpha = sm.prow[buf][ri], pr0 = sm.prow[buf][g], pr1 = sm.prow[buf][g + 8];
-  const double sp = col_total<MW>(sm.red[buf], ri, t);
-  const double s0 = col_total<MW>(sm.red[buf], g, t);
-  const double s1 = col_total<MW>(sm.red[buf], g + 8, t);
+  ColStep<K> c;
+  double pr[K::CN], s[K::CN];
+  const double alpha = sm.prow[buf][ri];
+#pragma unroll
+  for (int cs = 0; cs < K::CN; cs++) pr[cs] = sm.prow[buf][g + 8 * cs];
+  const double sp = col_total<K::MW>(sm.red[buf], ri, t);
+#pragma unroll
+  for (int cs = 0; cs < K::CN; cs++) s[cs] = col_total<K::MW>(sm.red[buf], g + 8 * cs, t);
   c.rf = reflector(sp, alpha);
   // v_I^T a_c = a_Ic + scale d_c.
-  c.w0 = fma(c.rf.scale, s0, pr0);
-  c.w1 = fma(c.rf.scale, s1, pr1);
+#pragma unroll
+  for (int cs = 0; cs < K::CN; cs++) c.w[cs] = fma(c.rf.scale, s[cs], pr[cs]);
   return c;
 }
 
 // The column loop of a row warp.
 template <class K>
-BSOFI_DEVINL void factor_rows(double (&a)[K::NI][2][2], ChainSmem<K::MW>& sm, int w, int ab8,
+BSOFI_DEVINL void factor_rows(double (&a)[K::NI][K::CN][2], ChainSmem<K::MW>& sm, int w, int ab8,
                               int nb, int g, int t, int warp) {
-  constexpr int MW = K::MW;
-  const int c0 = col_of(g), c1 = c0 + 8;
-  double x[K::NI][2];
-  double d0, d1;
-  row_first<K>(a, x, t, d0, d1);
-  put_partials<MW>(sm.red[0], d0, d1, g, t, warp);
+  const int c0 = col_of(g);
+  double x[K::NI][2], d[K::CN];
+  row_first<K>(a, x, t, d);
+  put_partials<K>(sm.red[0], d, g, t, warp);
   int I = 0;
-  auto step = [&](auto upd0, auto csu, auto csd) {
+  auto step = [&](auto csu, auto csd) {
     bar_col<K::CT>();
-    const ColStep c = col_step<MW>(sm, I, g, t);
-    const double f0 = c0 > I ? c.rf.q * c.w0 : 0.0, f1 = c1 > I ? c.rf.q * c.w1 : 0.0;
+    const ColStep<K> c = col_step<K>(sm, I, g, t);
+    double f[K::CN];
+#pragma unroll
+    for (int cs = 0; cs < K::CN; cs++) f[cs] = c0 + 8 * cs > I ? c.rf.q * c.w[cs] : 0.0;
     const int sd = group_of((I + 1) & 7) * 4 + t;
-    row_pass<K, upd0.value != 0, csu.value, csd.value>(a, x, f0, f1, sd, ab8, nb, warp, d0, d1);
-    put_partials<MW>(sm.red[(I + 1) & 1], d0, d1, g, t, warp);
+    row_pass<K, csu.value, csd.value>(a, x, f, sd, ab8, nb, warp, d);
+    put_partials<K>(sm.red[(I + 1) & 1], d, g, t, warp);
   };
   using Z = std::integral_constant<int, 0>;
   using O = std::integral_constant<int, 1>;
   const int last = w - 1;
 #pragma unroll 1
-  for (; I < min(last, 7); I++) step(O{}, Z{}, Z{});
-  if (I < last) {  // I = 7
-    step(Z{}, Z{}, O{});
-    I++;
+  for (; I < min(last, 7); I++) step(Z{}, Z{});
+  if constexpr (K::CN == 2) {
+    if (I < last) {  // I = 7
+      step(O{}, O{});
+      I++;
 #pragma unroll 1
-    for (; I < last; I++) step(Z{}, O{}, O{});
+      for (; I < last; I++) step(O{}, O{});
+    }
   }
   bar_col<K::CT>();  // the last column's sums are there
   bar_col<K::CT>();  // and its scale
 }
 
-// The top warp's 16 pivot rows (blocks 0, 1 in a[0], a[1]): update by pivot
-// column I (half CSU; rows below I; row I by v_I = 1, its pivot entry becomes
-// beta).
+// The top warp's LW pivot rows (blocks 0.. in a[0]..): update by pivot column I
+// (set CSU; rows below I; row I by v_I = 1, its pivot entry becomes beta).
 template <class K, int CSU>
-BSOFI_DEVINL void top_update(double (&a)[K::NI][2][2], const double (&x)[2][2], const Refl& rf,
-                             double F0, double F1, int I, int g, int t) {
+BSOFI_DEVINL void top_update(double (&a)[K::NI][K::CN][2], const double (&x)[K::CN][2],
+                             const Refl& rf, const double (&F)[K::CN], int I, int g, int t) {
 #pragma unroll
-  for (int b = CSU; b < 2; b++)
+  for (int b = CSU; b < K::CN; b++)
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       const int row = 8 * b + 2 * t + h;
       const double v = row == I ? 1.0 : x[b][h] * rf.scale;
-      if (CSU == 0) a[b][0][h] = fma(-v, F0, a[b][0][h]);
-      a[b][1][h] = fma(-v, F1, a[b][1][h]);
+#pragma unroll
+      for (int cs = CSU; cs < K::CN; cs++) a[b][cs][h] = fma(-v, F[cs], a[b][cs][h]);
       if (b == CSU && row == I && g == group_of(I & 7)) a[b][CSU][h] = rf.beta;
     }
 }
 
-// Dot products with column J (half CSD) over rows below J, and row J to prow.
+// Dot products with column J (set CSD) over rows below J, and row J to prow.
 template <class K, int CSD>
-BSOFI_DEVINL void top_dots(const double (&a)[K::NI][2][2], double (&x)[2][2], int J, int g, int t,
-                           double* prow, double& d0, double& d1) {
+BSOFI_DEVINL void top_dots(const double (&a)[K::NI][K::CN][2], double (&x)[K::CN][2], int J, int g,
+                           int t, double* prow, double (&d)[K::CN]) {
   const int src = group_of(J & 7) * 4 + t;
-  d0 = d1 = 0.0;
 #pragma unroll
-  for (int b = CSD; b < 2; b++)
+  for (int cs = 0; cs < K::CN; cs++) d[cs] = 0.0;
+#pragma unroll
+  for (int b = CSD; b < K::CN; b++)
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       const int row = 8 * b + 2 * t + h;
       const double xs = shfl_d(a[b][CSD][h], src);
       x[b][h] = row > J ? xs : 0.0;
-      d0 = fma(x[b][h], a[b][0][h], d0);
-      d1 = fma(x[b][h], a[b][1][h], d1);
+#pragma unroll
+      for (int cs = 0; cs < K::CN; cs++) d[cs] = fma(x[b][h], a[b][cs][h], d[cs]);
       if (b == CSD && row == J) {
-        prow[g] = a[b][0][h];
-        prow[g + 8] = a[b][1][h];
+#pragma unroll
+        for (int cs = 0; cs < K::CN; cs++) prow[g + 8 * cs] = a[b][cs][h];
       }
     }
 }
 
 // The column loop of the top warp.
 template <class K>
-BSOFI_DEVINL void factor_top(double (&a)[K::NI][2][2], ChainSmem<K::MW>& sm, int w, int g, int t,
-                             double* tau) {
-  constexpr int MW = K::MW;
-  const int c0 = col_of(g), c1 = c0 + 8;
-  double x[2][2], d0, d1, sc0 = 0.0, sc1 = 0.0;
-  top_dots<K, 0>(a, x, 0, g, t, sm.prow[0], d0, d1);
-  put_partials<MW>(sm.red[0], d0, d1, g, t, K::FW);
+BSOFI_DEVINL void factor_top(double (&a)[K::NI][K::CN][2], ChainSmem<K::MW>& sm, int w, int g,
+                             int t, double* tau) {
+  const int c0 = col_of(g);
+  double x[K::CN][2], d[K::CN], sc[K::CN];
+#pragma unroll
+  for (int cs = 0; cs < K::CN; cs++) sc[cs] = 0.0;
+  top_dots<K, 0>(a, x, 0, g, t, sm.prow[0], d);
+  put_partials<K>(sm.red[0], d, g, t, K::FW);
   int I = 0;
   auto step = [&](auto csu, auto csd, auto dot) {
     bar_col<K::CT>();
-    const ColStep c = col_step<MW>(sm, I, g, t);
-    const double F0 = c0 > I ? c.rf.tau * c.w0 : 0.0, F1 = c1 > I ? c.rf.tau * c.w1 : 0.0;
-    top_update<K, csu.value>(a, x, c.rf, F0, F1, I, g, t);
+    const ColStep<K> c = col_step<K>(sm, I, g, t);
+    double F[K::CN];
+#pragma unroll
+    for (int cs = 0; cs < K::CN; cs++) F[cs] = c0 + 8 * cs > I ? c.rf.tau * c.w[cs] : 0.0;
+    top_update<K, csu.value>(a, x, c.rf, F, I, g, t);
     if (dot.value) {
-      top_dots<K, csd.value>(a, x, I + 1, g, t, sm.prow[(I + 1) & 1], d0, d1);
-      put_partials<MW>(sm.red[(I + 1) & 1], d0, d1, g, t, K::FW);
+      top_dots<K, csd.value>(a, x, I + 1, g, t, sm.prow[(I + 1) & 1], d);
+      put_partials<K>(sm.red[(I + 1) & 1], d, g, t, K::FW);
     }
     // v_j^T v_I of the finished columns j < I (both unscaled in registers,
     // row I of v_I is 1) for the T warp.
     if (t == 0) {
       double* v = sm.vtv[I & 1];
-      v[c0] = c0 < I ? sc0 * c.w0 : 0.0;
-      v[c1] = c1 < I ? sc1 * c.w1 : 0.0;
+#pragma unroll
+      for (int cs = 0; cs < K::CN; cs++)
+        v[c0 + 8 * cs] = c0 + 8 * cs < I ? sc[cs] * c.w[cs] : 0.0;
       if (g == 0) {
         v[16] = c.rf.tau;
         tau[I] = c.rf.tau;
         sm.sc[I] = c.rf.scale;
       }
     }
-    if (I == c0) sc0 = c.rf.scale;
-    if (I == c1) sc1 = c.rf.scale;
+#pragma unroll
+    for (int cs = 0; cs < K::CN; cs++)
+      if (I == c0 + 8 * cs) sc[cs] = c.rf.scale;
   };
   using Z = std::integral_constant<int, 0>;
   using O = std::integral_constant<int, 1>;
   const int last = w - 1;
 #pragma unroll 1
   for (; I < min(last, 7); I++) step(Z{}, Z{}, O{});
-  if (I < last) {  // I = 7
-    step(Z{}, O{}, O{});
-    I++;
+  if constexpr (K::CN == 2) {
+    if (I < last) {  // I = 7
+      step(Z{}, O{}, O{});
+      I++;
 #pragma unroll 1
-    for (; I < last; I++) step(O{}, O{}, O{});
+      for (; I < last; I++) step(O{}, O{}, O{});
+    }
+    if (I < 8) step(Z{}, Z{}, Z{});
+    else step(O{}, O{}, Z{});
+  } else {
+    step(Z{}, Z{}, Z{});
   }
-  if (I < 8) step(Z{}, Z{}, Z{});
-  else step(O{}, O{}, Z{});
   bar_col<K::CT>();
 }
 
 // The T warp: column I of T one barrier behind the factorization (LAPACK
 // dlarft): T(0:I,I) = -tau_I T(0:I,0:I) V(:,0:I)^T v_I.  Lane 4 g + t holds
-// rows g and g+8 of columns t, t+4, t+8, t+12.
-BSOFI_DEVINL void t_column(double (&T)[2][4], const double* vtv, int I, int g, int t) {
-  double r0 = 0.0, r1 = 0.0;
+// rows g (and g+8) of columns t, t+4, ..
+template <int CN>
+BSOFI_DEVINL void t_column(double (&T)[CN][2 * CN], const double* vtv, int I, int g, int t) {
+  double r[CN];
 #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const double gb = vtv[t + 4 * q];
-    r0 = fma(T[0][q], gb, r0);
-    r1 = fma(T[1][q], gb, r1);
+  for (int cs = 0; cs < CN; cs++) {
+    r[cs] = 0.0;
+#pragma unroll
+    for (int q = 0; q < 2 * CN; q++) r[cs] = fma(T[cs][q], vtv[t + 4 * q], r[cs]);
   }
   const double tau = vtv[16];
-  r0 = quad_sum(r0);
-  r1 = quad_sum(r1);
-  const double v0 = g == I ? tau : (g < I ? -tau * r0 : 0.0);
-  const double v1 = g + 8 == I ? tau : (g + 8 < I ? -tau * r1 : 0.0);
 #pragma unroll
-  for (int q = 0; q < 4; q++)
-    if (I == t + 4 * q) {
-      T[0][q] = v0;
-      T[1][q] = v1;
-    }
+  for (int cs = 0; cs < CN; cs++) {
+    const double s = quad_sum(r[cs]);
+    const double v = g + 8 * cs == I ? tau : (g + 8 * cs < I ? -tau * s : 0.0);
+#pragma unroll
+    for (int q = 0; q < 2 * CN; q++)
+      if (I == t + 4 * q) T[cs][q] = v;
+  }
 }
 
 // ------------------------------------------------------------ block update
@@ -604,30 +701,51 @@ BSOFI_DEVINL int widx(int c, int j) { return c * 16 + (j ^ ((c & 4) << 1)); }
 // col_of(g) + 8 and (its B operand having V's columns in the lane groups'
 // order) columns 8 jt + t, 8 jt + t + 4.  The fragments' K index t stands for
 // j = 8 kk + 2t and t + 4 for 8 kk + 2t + 1.  Two barriers among the MW warps.
-template <int MW>
-BSOFI_DEVINL void reduce_w(double (&acc)[2][4], double (&fr)[2][4], double* part, ChainSmem<MW>& sm,
-                           int g, int t, int warp) {
-  // (W^T T): T is upper triangular, so columns 0..7 need only rows 0..7.
-  double o[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
-  dmma_16x8x8(o[0], acc[0][0], acc[0][2], acc[0][1], acc[0][3], sm.T[t][g], sm.T[t + 4][g]);
-  dmma_16x8x8(o[1], acc[0][0], acc[0][2], acc[0][1], acc[0][3], sm.T[t][g + 8],
-              sm.T[t + 4][g + 8]);
-  dmma_16x8x8(o[1], acc[1][0], acc[1][2], acc[1][1], acc[1][3], sm.T[8 + t][g + 8],
-              sm.T[12 + t][g + 8]);
-  double* mine = part + warp * 256;
+//
+// With 8-wide leaves the same with one tile, m8n8k4 and its K index t for j = t
+// and t + 4, or 2t and 2t + 1 in the fragments.
+template <int CN>
+BSOFI_DEVINL void mma_w(double (&acc)[2 * CN], const double (&c)[CN][2], double v0, double v1) {
+  if constexpr (CN == 2) {
+    dmma_16x8x8(acc, c[0][0], c[1][0], c[0][1], c[1][1], v0, v1);
+  } else {
+    dmma_8x8x4(acc, c[0][0], v0);
+    dmma_8x8x4(acc, c[0][1], v1);
+  }
+}
+
+template <int MW, int CN>
+BSOFI_DEVINL void reduce_w(double (&acc)[CN][2 * CN], double (&fr)[CN][2 * CN], double* part,
+                           ChainSmem<MW>& sm, int g, int t, int warp) {
+  constexpr int E = 64 * CN * CN;  // elements of W
+  double* mine = part + warp * E;
   const int c0 = col_of(g);
+  if constexpr (CN == 2) {
+    // (W^T T): T is upper triangular, so columns 0..7 need only rows 0..7.
+    double o[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+    dmma_16x8x8(o[0], acc[0][0], acc[0][2], acc[0][1], acc[0][3], sm.T[t][g], sm.T[t + 4][g]);
+    dmma_16x8x8(o[1], acc[0][0], acc[0][2], acc[0][1], acc[0][3], sm.T[t][g + 8],
+                sm.T[t + 4][g + 8]);
+    dmma_16x8x8(o[1], acc[1][0], acc[1][2], acc[1][1], acc[1][3], sm.T[8 + t][g + 8],
+                sm.T[12 + t][g + 8]);
 #pragma unroll
-  for (int jt = 0; jt < 2; jt++)
+    for (int jt = 0; jt < 2; jt++)
 #pragma unroll
-    for (int h = 0; h < 2; h++)
-      *reinterpret_cast<double2*>(mine + widx(c0 + 8 * h, 8 * jt + 2 * t)) =
-          make_double2(o[jt][2 * h], o[jt][2 * h + 1]);
+      for (int h = 0; h < 2; h++)
+        *reinterpret_cast<double2*>(mine + widx(c0 + 8 * h, 8 * jt + 2 * t)) =
+            make_double2(o[jt][2 * h], o[jt][2 * h + 1]);
+  } else {
+    double o[2] = {0.0, 0.0};
+    dmma_8x8x4(o, acc[0][0], sm.T[t][g]);
+    dmma_8x8x4(o, acc[0][1], sm.T[t + 4][g]);
+    *reinterpret_cast<double2*>(mine + c0 * 8 + 2 * t) = make_double2(o[0], o[1]);
+  }
   bar_main<32 * MW>();
 #pragma unroll
-  for (int e = threadIdx.x; e < 256; e += 32 * MW) {
+  for (int e = threadIdx.x; e < E; e += 32 * MW) {
     double s[MW];
 #pragma unroll
-    for (int k = 0; k < MW; k++) s[k] = part[k * 256 + e];
+    for (int k = 0; k < MW; k++) s[k] = part[k * E + e];
 #pragma unroll
     for (int m = MW / 2; m > 0; m /= 2)
 #pragma unroll
@@ -635,107 +753,182 @@ BSOFI_DEVINL void reduce_w(double (&acc)[2][4], double (&fr)[2][4], double* part
     sm.W[e] = -s[0];
   }
   bar_main<32 * MW>();
+  if constexpr (CN == 2) {
 #pragma unroll
-  for (int kk = 0; kk < 2; kk++)
+    for (int kk = 0; kk < 2; kk++)
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const double2 v =
-          *reinterpret_cast<const double2*>(sm.W + widx(c0 + 8 * h, 8 * kk + 2 * t));
-      fr[kk][h] = v.x;
-      fr[kk][2 + h] = v.y;
-    }
+      for (int h = 0; h < 2; h++) {
+        const double2 v =
+            *reinterpret_cast<const double2*>(sm.W + widx(c0 + 8 * h, 8 * kk + 2 * t));
+        fr[kk][h] = v.x;
+        fr[kk][2 + h] = v.y;
+      }
+  } else {
+    const double2 v = *reinterpret_cast<const double2*>(sm.W + c0 * 8 + 2 * t);
+    fr[0][0] = v.x;
+    fr[0][1] = v.y;
+  }
 }
 
 // C^T += fr V^T for the 8-row block at row r0 of V in shared memory.
-BSOFI_DEVINL void update_block(double (&c)[2][2], const double (&fr)[2][4], const double* sV, int SV,
-                               int r0, int g, int t) {
-  double d[4] = {c[0][0], c[0][1], c[1][0], c[1][1]};
+template <int CN>
+BSOFI_DEVINL void update_block(double (&c)[CN][2], const double (&fr)[CN][2 * CN],
+                               const double* sV, int SV, int r0, int g, int t) {
+  if constexpr (CN == 2) {
+    double d[4] = {c[0][0], c[0][1], c[1][0], c[1][1]};
 #pragma unroll
-  for (int kk = 0; kk < 2; kk++)
-    dmma_16x8x8(d, fr[kk][0], fr[kk][1], fr[kk][2], fr[kk][3],
-                sV[sidx(r0 + g, 8 * kk + 2 * t, SV)], sV[sidx(r0 + g, 8 * kk + 2 * t + 1, SV)]);
-  c[0][0] = d[0];
-  c[0][1] = d[1];
-  c[1][0] = d[2];
-  c[1][1] = d[3];
+    for (int kk = 0; kk < 2; kk++)
+      dmma_16x8x8(d, fr[kk][0], fr[kk][1], fr[kk][2], fr[kk][3],
+                  sV[sidx(r0 + g, 8 * kk + 2 * t, SV)], sV[sidx(r0 + g, 8 * kk + 2 * t + 1, SV)]);
+    c[0][0] = d[0];
+    c[0][1] = d[1];
+    c[1][0] = d[2];
+    c[1][1] = d[3];
+  } else {
+    dmma_8x8x4(c[0], fr[0][0], sV[sidx(r0 + g, 2 * t, SV)]);
+    dmma_8x8x4(c[0], fr[0][1], sV[sidx(r0 + g, 2 * t + 1, SV)]);
+  }
 }
 
 // ------------------------------------------------------------ the chain CTA
-// The helper warps: wait for the next tile and stage it while the leaf
-// is being factored, build T; store and publish the leaf while the next tile
-// is being updated.
+// The reflectors below the pivot rows to global memory, by W warps of which this
+// is warp w (the pivot rows and, in short panels, all of V are stored by the
+// warps that hold them).
+template <class K, int W>
+BSOFI_DEVINL void store_leaf(const ChainStep& z, const double* sV, int SV, int lane, int w) {
+  if constexpr (K::BULK) {
+    const int r0 = z.ab + K::LW;
+    if (pair_aligned(z.P, z.ldp) && ((z.rows - r0) & 1) == 0) {
+      if (w == 0 && lane == 0 && z.rows > r0) {
+        for (int c = 0; c < z.f.w; c++)
+          bulk_store(z.P + cm(r0, c, z.ldp), sV + sidx(r0, c, SV), z.rows - r0);
+        bulk_store_wait();
+        fence_proxy();
+      }
+    } else {
+#pragma unroll 1
+      for (int c = w; c < z.f.w; c += W) {
+        double* col = z.P + cm(0, c, z.ldp);
+#pragma unroll 4
+        for (int r = r0 + lane; r < z.rows; r += 32) __stcg(col + r, sV[sidx(r, c, SV)]);
+      }
+    }
+  }
+}
+
+// The helper warps: wait for the next tile and stage it while the leaf is being
+// factored; the last one (the T warp) builds T.  One side or the other stores
+// and publishes the leaf.
 template <class K>
 BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const double* sV, double* sC,
                                int SV, ChainSmem<K::MW>& sm) {
   const int ht = threadIdx.x - K::MT, lane = threadIdx.x & 31, hw = ht >> 5;
   const int n = g.n, SC = SV + 16, capc = SC - 2;
   uint32_t phase = 0;
-  constexpr int LW = K::HW - 1;  // loading warps; the last one builds T
-  if (hw == LW) {
+  constexpr int LD = K::HW - 1;  // loading warps; the last one builds T
+  if (hw == LD) {
     const int gq = lane >> 2, t = lane & 3;
     for (int s = st.s_begin; s < st.s_end; s++) {
       const Leaf f = sm.step[s & 1].f;
-      double T[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+      double T[K::CN][2 * K::CN] = {};
       for (int I = 0; I <= f.w; I++) {
         bar_col<K::CT>();
-        if (I > 0) t_column(T, sm.vtv[(I - 1) & 1], I - 1, gq, t);
+        if (I > 0) t_column<K::CN>(T, sm.vtv[(I - 1) & 1], I - 1, gq, t);
       }
       double* Tout = st.T + ((long long)f.k * st.maxleaves + f.l) * 256;
 #pragma unroll
-      for (int r = 0; r < 2; r++)
+      for (int r = 0; r < K::CN; r++)
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
+        for (int q = 0; q < 2 * K::CN; q++) {
           const int i = gq + 8 * r, j = t + 4 * q;
           sm.T[i][j] = T[r][q];
           Tout[i + 16 * j] = T[r][q];
         }
-      bar_all<K::THREADS>();
-      if (!sm.flag) return;
+      if constexpr (K::EARLY) {
+        bar_ready_arrive<K::THREADS>();
+        bar_v<K::CT>();
+        store_leaf<K, 1>(sm.step[s & 1], sV, SV, lane, 0);
+        __syncwarp();
+        if (lane == 0) {
+          __threadfence();
+          red_release_add(st.factored + s, 1);
+        }
+      } else {
+        bar_ready<K::THREADS>();
+      }
       if (lane == 0 && s + 1 < st.s_end) sm.step[(s + 1) & 1] = chain_step(g, st, s + 1);
-      bar_all<K::THREADS>();
+      bar_done<K::THREADS>();
+      if (!sm.ok[s & 1]) return;
     }
     return;
   }
   for (int s = st.s_begin; s < st.s_end; s++) {
     const ChainStep& z = sm.step[s & 1];
-    if (ht == 0)
-      sm.flag = !z.next || wait_geq(st, st.cnt + tile_id(g, z.m2, z.t2), s - z.lo2) ? 1 : 0;
+    int& ok = sm.ok[s & 1];
+    if (ht == 0) ok = !z.next || wait_geq(st, st.cnt + tile_id(g, z.m2, z.t2), s - z.lo2) ? 1 : 0;
     {
-      bar_help<32 * LW>();
-      if (z.next && sm.flag) {
+      bar_help<32 * LD>();
+      if (z.next && ok) {
         // Rows [ab, rows) of the tile, then (fresh) the n rows below the panel
         // at shared rows 8 nb, 8 nb + 1, .. (mod capc; the tile's own rows
         // above ab leave room).
-        const bool vec = pair_aligned(z.C, z.ldc) && (n & 1) == 0;
         const int f0 = 8 * z.nb, q0 = min(n, capc - f0);
-        if (vec && K::BULK) {
+        const double* F = z.C + 2 * n;
+        const bool vec = pair_aligned(z.C, z.ldc) &&
+                         (K::EARLY ? ((z.rows | (z.fresh ? n : 0)) & 1) == 0 : (n & 1) == 0);
+        if (K::BULK && (vec || K::EARLY)) {
+          // The spans of column c: f(dst, src, elements).
+          auto spans = [&](int c, auto f) {
+            const long long at = cm(0, c, z.ldc);
+            f(sC + sidx(z.ab, c, SC), z.C + at + z.ab, z.rows - z.ab);
+            if (z.fresh) {
+              f(sC + sidx(f0, c, SC), F + at, q0);
+              if (n > q0) f(sC + sidx(0, c, SC), F + at + q0, n - q0);
+            }
+          };
           if (ht == 0) {
+            int total = z.w2 * (z.rows - z.ab + (z.fresh ? n : 0));
+            if (K::EARLY && !vec) {
+              total = 0;
+              for (int c = 0; c < z.w2; c++)
+                spans(c, [&](double*, const double* src, int cnt) { total += span_bulk(src, cnt); });
+            }
             fence_proxy();
-            tc::mbar_arrive_expect_tx(&sm.bar, 8 * z.w2 * (z.rows - z.ab + (z.fresh ? n : 0)));
-            for (int c = 0; c < z.w2; c++) {
-              const double* col = z.C + cm(0, c, z.ldc);
-              bulk_load(sC + sidx(z.ab, c, SC), col + z.ab, z.rows - z.ab, &sm.bar);
+            tc::mbar_arrive_expect_tx(&sm.bar, 8 * total);
+            for (int c = 0; c < z.w2; c++)
+              spans(c, [&](double* dst, const double* src, int cnt) {
+                if (!K::EARLY || vec) bulk_load(dst, src, cnt, &sm.bar);
+                else span_issue(dst, src, cnt, &sm.bar);
+              });
+          }
+        }
+        if constexpr (K::EARLY) {
+          if (!vec) {
+            if (ht == 0 && !bulk_wait(&sm.bar, phase, st.err)) ok = 0;
+            bar_help<32 * LD>();
+#pragma unroll 1
+            for (int c = hw; c < z.w2; c += LD) {
+              const long long at = cm(0, c, z.ldc);
+              span_finish(sC + sidx(z.ab, c, SC), z.C + at + z.ab, z.rows - z.ab, lane);
               if (z.fresh) {
-                bulk_load(sC + sidx(f0, c, SC), col + 2 * n, q0, &sm.bar);
-                if (n > q0) bulk_load(sC + sidx(0, c, SC), col + 2 * n + q0, n - q0, &sm.bar);
+                span_finish(sC + sidx(f0, c, SC), F + at, q0, lane);
+                if (n > q0) span_finish(sC + sidx(0, c, SC), F + at + q0, n - q0, lane);
               }
             }
           }
-        }
-        if (!vec) {
+        } else if (!vec) {
           constexpr int NC = 16 / K::LOADS;
 #pragma unroll 1
-          for (int c = hw; c < z.w2; c += NC * LW) {
-            copy_cols<NC, K::LOADS>(sC, SC, z.C, z.ldc, c, LW, z.w2, z.ab, z.rows, lane);
+          for (int c = hw; c < z.w2; c += NC * LD) {
+            copy_cols<NC, K::LOADS>(sC, SC, z.C, z.ldc, c, LD, z.w2, z.ab, z.rows, lane);
             if (z.fresh) {
-              const double* F = z.C + 2 * n;
-              copy_cols<NC, K::LOADS>(sC + f0, SC, F, z.ldc, c, LW, z.w2, 0, q0, lane);
-              copy_cols<NC, K::LOADS>(sC - q0, SC, F, z.ldc, c, LW, z.w2, q0, n, lane);
+              copy_cols<NC, K::LOADS>(sC + f0, SC, F, z.ldc, c, LD, z.w2, 0, q0, lane);
+              copy_cols<NC, K::LOADS>(sC - q0, SC, F, z.ldc, c, LD, z.w2, q0, n, lane);
             }
           }
         }
 #pragma unroll 1
-        for (int c = hw; c < 16; c += LW) {
+        for (int c = hw; c < K::LW; c += LD) {
           const double* col = z.C + cm(0, c, z.ldc);
           if (c >= z.w2) {
             for (int r = z.ab + lane; r < 8 * z.nb; r += 32) sC[sidx(r, c, SC)] = 0.0;
@@ -758,69 +951,57 @@ BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const dou
         if (!K::BULK) {
           cp_async_commit();
           cp_async_wait<0>();
-        } else if (vec && ht == 0) {
-          if (!bulk_wait(&sm.bar, phase, st.err)) sm.flag = 0;
+        } else if (vec || K::EARLY) {
+          if (vec && ht == 0 && !bulk_wait(&sm.bar, phase, st.err)) ok = 0;
           phase ^= 1;
         }
       }
     }
-    bar_all<K::THREADS>();
-    if (!sm.flag) return;
-    // The reflectors below the pivot rows to global memory.
+    bar_ready<K::THREADS>();
     if (ht == 0) st.timeline[4 * s + 3] = gtimer();
-    if constexpr (K::BULK) {
-      const bool vec = pair_aligned(z.P, z.ldp);
-      const int r0 = z.ab + 16;
-      if (vec && ((z.rows - r0) & 1) == 0) {
-        if (ht == 0 && z.rows > r0) {
-          for (int c = 0; c < z.f.w; c++)
-            bulk_store(z.P + cm(r0, c, z.ldp), sV + sidx(r0, c, SV), z.rows - r0);
-          bulk_store_wait();
-          fence_proxy();
-        }
-      } else {
-#pragma unroll 1
-        for (int c = hw; c < z.f.w; c += LW) {
-          double* col = z.P + cm(0, c, z.ldp);
-#pragma unroll 4
-          for (int r = r0 + lane; r < z.rows; r += 32) __stcg(col + r, sV[sidx(r, c, SV)]);
+    const bool go = ok != 0;
+    if constexpr (!K::EARLY) {
+      if (go) {
+        store_leaf<K, LD>(z, sV, SV, lane, hw);
+        if constexpr (K::BULK) bar_help<32 * LD>();
+        if (ht == 0) {
+          __threadfence();
+          red_release_add(st.factored + s, 1);
         }
       }
     }
-    if constexpr (K::BULK) bar_help<32 * LW>();
-    if (ht == 0) {
-      __threadfence();
-      red_release_add(st.factored + s, 1);
-    }
-    bar_all<K::THREADS>();
+    bar_done<K::THREADS>();
+    if (!go) return;
   }
 }
 
 template <class K>
 BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV, double* part,
                              double* sC, int SV, ChainSmem<K::MW>& sm) {
-  constexpr int FW = K::FW, NI = K::NI, MW = K::MW, MT = K::MT;
+  constexpr int FW = K::FW, NI = K::NI, MW = K::MW, MT = K::MT, CN = K::CN;
   // (The shuffle tells the compiler that the warp index is uniform.)
   const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int gq = lane >> 2, t = lane & 3, gc = col_of(gq);
   const bool top = warp == FW;
   const int n = g.n, SC = SV + 16, capc = SC - 2;
   // Slot i of this warp is 8-row block bb + i bs of the panel.
-  double a[NI][2][2];
+  double a[NI][CN][2];
 #pragma unroll
-  for (int i = 0; i < NI; i++) a[i][0][0] = a[i][0][1] = a[i][1][0] = a[i][1][1] = 0.0;
+  for (int i = 0; i < NI; i++)
+#pragma unroll
+    for (int cs = 0; cs < CN; cs++) a[i][cs][0] = a[i][cs][1] = 0.0;
   {
     const Leaf f = leaf_of(g, st.s_begin);
     const int base = leaf_base(g, f), ab8 = (f.j0 - base) / 8, rows = 2 * n - base;
     long long ld;
-    const double* P = mat_ptr(g, st, (long long)f.k * n + base, f.m, f.t * 16, ld);
+    const double* P = mat_ptr(g, st, (long long)f.k * n + base, f.m, f.t * g.NB, ld);
     const bool vec = pair_aligned(P, ld);
 #pragma unroll
     for (int i = 0; i < NI; i++) {
-      const int b = top ? ab8 + i : 2 + i * FW + warp;
-      if (top ? i >= 2 : b < ab8 + 2) continue;
+      const int b = top ? ab8 + i : CN + i * FW + warp;
+      if (top ? i >= CN : b < ab8 + CN) continue;
 #pragma unroll
-      for (int cs = 0; cs < 2; cs++) {
+      for (int cs = 0; cs < K::CN; cs++) {
         const int c = gc + 8 * cs;
         const double2 v = ld_pair(P + cm(0, c, ld), 8 * b + 2 * t, rows, c < f.w, vec);
         a[i][cs][0] = v.x;
@@ -834,8 +1015,8 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
     const bool next = z.next, fresh = z.fresh, trans = z.trans;
     double* C = z.C;
     const long long ldc = z.ldc;
-    const int blo = top ? ab8 : ab8 + 2, bhi = top ? min(nb, ab8 + 2) : nb;
-    const int bb = top ? ab8 : 2 + warp, bs = top ? 1 : FW;
+    const int blo = top ? ab8 : ab8 + CN, bhi = top ? min(nb, ab8 + CN) : nb;
+    const int bb = top ? ab8 : CN + warp, bs = top ? 1 : FW;
     {
       // ---- factor the leaf
       if (top) {
@@ -849,20 +1030,22 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
       }
       // ---- V to shared memory, the pivot rows (R and V) to global memory
       // (columns beyond the leaf's width are zero whatever their scale).
-      const double sc0 = gc < w ? sm.sc[gc] : 0.0, sc1 = gc + 8 < w ? sm.sc[gc + 8] : 0.0;
+      double sc[CN];
+#pragma unroll
+      for (int cs = 0; cs < K::CN; cs++) sc[cs] = gc + 8 * cs < w ? sm.sc[gc + 8 * cs] : 0.0;
       const bool vecp = pair_aligned(z.P, z.ldp);
       if (top) {
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < CN; i++) {
 #pragma unroll
-          for (int cs = 0; cs < 2; cs++) {
+          for (int cs = 0; cs < K::CN; cs++) {
             const int c = gc + 8 * cs, r = ab + 8 * i + 2 * t;
             double o[2], v[2];
 #pragma unroll
             for (int h = 0; h < 2; h++) {
               const double e = a[i][cs][h];
               const int d = 8 * i + 2 * t + h - c;  // row minus column of the leaf
-              o[h] = d > 0 ? e * (cs == 0 ? sc0 : sc1) : e;
+              o[h] = d > 0 ? e * sc[cs] : e;
               v[h] = d > 0 ? o[h] : ((d == 0 && c < w) ? 1.0 : 0.0);
               a[i][cs][h] = v[h];
             }
@@ -877,10 +1060,10 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
           const int b = bb + i * bs;
           if (b < blo || b >= bhi) continue;
 #pragma unroll
-          for (int cs = 0; cs < 2; cs++) {
+          for (int cs = 0; cs < K::CN; cs++) {
             const int c = gc + 8 * cs, r = 8 * b + 2 * t;
 #pragma unroll
-            for (int h = 0; h < 2; h++) a[i][cs][h] *= cs == 0 ? sc0 : sc1;
+            for (int h = 0; h < 2; h++) a[i][cs][h] *= sc[cs];
             if constexpr (!K::BULK)
               st_pair(z.P + cm(0, c, z.ldp), r, rows, c < w, vecp, a[i][cs][0], a[i][cs][1]);
             *reinterpret_cast<double2*>(sV + sidx(r, c, SV)) =
@@ -889,15 +1072,19 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
         }
       }
       if constexpr (K::BULK) tc::fence_proxy_async_smem();  // V is stored to global memory by bulk copies
+      if constexpr (K::EARLY) bar_v_arrive<K::CT>();
     }
-    bar_all<K::THREADS>();
-    if (!sm.flag) return;
+    bar_ready<K::THREADS>();
+    if (!sm.ok[s & 1]) {
+      bar_done<K::THREADS>();
+      return;
+    }
     if (next) {
       // ---- leaf s on the tile of leaf s+1.  That is the tile's last update
       // and only this CTA reads the tile next, so it stays in registers; its
       // rows above the next leaf are final and go to global memory.
-      double c[NI][2][2];
-      double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+      double c[NI][CN][2];
+      double acc[CN][2 * CN] = {};
       const bool vec = pair_aligned(C, ldc);
       constexpr int GS = K::GS;
 #pragma unroll
@@ -905,14 +1092,16 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
         const int ia = q * GS, ie = (ia + GS < NI ? ia + GS : NI);
         const bool any = bb + (ie - 1) * bs >= blo && bb + ia * bs < bhi;
 #pragma unroll
-        for (int i = ia; i < ie; i++) c[i][0][0] = c[i][0][1] = c[i][1][0] = c[i][1][1] = 0.0;
+        for (int i = ia; i < ie; i++)
+#pragma unroll
+          for (int cs = 0; cs < K::CN; cs++) c[i][cs][0] = c[i][cs][1] = 0.0;
         if (!any) continue;
 #pragma unroll
         for (int i = ia; i < ie; i++) {
           const int b = bb + i * bs, r = 8 * b + 2 * t;
           const bool live = b >= blo && b < bhi;
 #pragma unroll
-          for (int cs = 0; cs < 2; cs++) {
+          for (int cs = 0; cs < K::CN; cs++) {
             const int cc = gc + 8 * cs;
             double2 v = make_double2(0.0, 0.0);
             if (live) v = *reinterpret_cast<const double2*>(sC + sidx(r, cc, SC));
@@ -924,9 +1113,7 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
 #pragma unroll
           for (int i = ia; i < ie; i++)
 #pragma unroll
-            for (int jt = 0; jt < 2; jt++)
-              dmma_16x8x8(acc[jt], c[i][0][0], c[i][1][0], c[i][0][1], c[i][1][1], a[i][jt][0],
-                          a[i][jt][1]);
+            for (int jt = 0; jt < CN; jt++) mma_w<CN>(acc[jt], c[i], a[i][jt][0], a[i][jt][1]);
         }
       }
       if constexpr (!K::VREG) {
@@ -935,14 +1122,14 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
           const int b = bb + i * bs, r = 8 * b + 2 * t;
           if (b < blo || b >= bhi) continue;
 #pragma unroll
-          for (int jt = 0; jt < 2; jt++) {
+          for (int jt = 0; jt < CN; jt++) {
             const double2 v = *reinterpret_cast<const double2*>(sV + sidx(r, gc + 8 * jt, SV));
-            dmma_16x8x8(acc[jt], c[i][0][0], c[i][1][0], c[i][0][1], c[i][1][1], v.x, v.y);
+            mma_w<CN>(acc[jt], c[i], v.x, v.y);
           }
         }
       }
-      double fr[2][4];
-      reduce_w<MW>(acc, fr, part, sm, gq, t, warp);
+      double fr[CN][2 * CN];
+      reduce_w<MW, CN>(acc, fr, part, sm, gq, t, warp);
       const bool keep_all = s + 1 == st.s_end;
 #pragma unroll
       for (int q = 0; q < K::NG; q++) {
@@ -951,7 +1138,7 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
         // (Slots of the group that are not live compute values nobody uses.)
 #pragma unroll
         for (int i = ia; i < ie; i++)
-          update_block(c[i], fr, sV, SV, 8 * min(bb + i * bs, nb - 1), gq, t);
+          update_block<CN>(c[i], fr, sV, SV, 8 * min(bb + i * bs, nb - 1), gq, t);
       }
       if (top || keep_all) {
 #pragma unroll
@@ -959,24 +1146,24 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
           const int b = bb + i * bs, r = 8 * b + 2 * t;
           if (b < blo || b >= bhi) continue;
 #pragma unroll
-          for (int cs = 0; cs < 2; cs++)
+          for (int cs = 0; cs < K::CN; cs++)
             st_pair(C + cm(0, gc + 8 * cs, ldc), r, rows, gc + 8 * cs < w2, vec, c[i][cs][0],
                     c[i][cs][1]);
         }
       }
       if (!trans) {
-        // Blocks ab8 + 2 and ab8 + 3 become the next leaf's pivot rows.
+        // Blocks ab8 + CN .. ab8 + 2 CN - 1 become the next leaf's pivot rows.
 #pragma unroll
         for (int i = 0; i < NI; i++) {
-          const int d = bb + i * bs - (ab8 + 2);
+          const int d = bb + i * bs - (ab8 + CN);
           const bool live = !top && d >= 0 && bb + i * bs < bhi;
 #pragma unroll
-          for (int cs = 0; cs < 2; cs++) {
-            if (live && d < 2)
+          for (int cs = 0; cs < K::CN; cs++) {
+            if (live && d < CN)
               *reinterpret_cast<double2*>(sm.top + (gc + 8 * cs) * 16 + 8 * d + 2 * t) =
                   make_double2(c[i][cs][0], c[i][cs][1]);
 #pragma unroll
-            for (int h = 0; h < 2; h++) a[i][cs][h] = live && d >= 2 ? c[i][cs][h] : 0.0;
+            for (int h = 0; h < 2; h++) a[i][cs][h] = live && d >= CN ? c[i][cs][h] : 0.0;
           }
         }
       } else {
@@ -986,7 +1173,7 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
           const int b = bb + i * bs;
           if (b < blo || b >= bhi) continue;
 #pragma unroll
-          for (int cs = 0; cs < 2; cs++)
+          for (int cs = 0; cs < K::CN; cs++)
             *reinterpret_cast<double2*>(sC + sidx(8 * b + 2 * t, gc + 8 * cs, SC)) =
                 make_double2(c[i][cs][0], c[i][cs][1]);
         }
@@ -994,14 +1181,14 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
         const int rows2 = fresh ? 2 * n : n;
 #pragma unroll
         for (int i = 0; i < NI; i++) {
-          const int b = top ? i : 2 + i * FW + warp;
+          const int b = top ? i : CN + i * FW + warp;
 #pragma unroll
-          for (int cs = 0; cs < 2; cs++)
+          for (int cs = 0; cs < K::CN; cs++)
 #pragma unroll
             for (int h = 0; h < 2; h++) {
               const int r = 8 * b + 2 * t + h, cc = gc + 8 * cs;
               double v = 0.0;
-              if ((!top || i < 2) && r < rows2 && cc < w2) {
+              if ((!top || i < CN) && r < rows2 && cc < w2) {
                 if (r < n) {
                   v = sC[sidx(n + r, cc, SC)];
                 } else {
@@ -1015,15 +1202,15 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
         }
       }
     }
-    bar_all<K::THREADS>();
+    bar_done<K::THREADS>();
     if (top) {
       if (next && !trans) {
 #pragma unroll
-        for (int i = 0; i < 2; i++)
+        for (int i = 0; i < CN; i++)
 #pragma unroll
-          for (int cs = 0; cs < 2; cs++) {
+          for (int cs = 0; cs < K::CN; cs++) {
             double2 v = make_double2(0.0, 0.0);
-            if (ab8 + 2 + i < nb)
+            if (ab8 + CN + i < nb)
               v = *reinterpret_cast<const double2*>(sm.top + (gc + 8 * cs) * 16 + 8 * i + 2 * t);
             a[i][cs][0] = v.x;
             a[i][cs][1] = v.y;
@@ -1038,7 +1225,7 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
 template <class K>
 BSOFI_DEVINL void worker(const BsofGeom& g, const BsofState& st, double* sV, double* part, int SV,
                          ChainSmem<K::MW>& sm) {
-  constexpr int MW = K::MW, MT = K::MT, NIW = K::NIW;
+  constexpr int MW = K::MW, MT = K::MT, NIW = K::NIW, CN = K::CN, LW = K::LW;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gq = lane >> 2, t = lane & 3, gc = col_of(gq);
   uint32_t phase = 0;
@@ -1065,20 +1252,20 @@ BSOFI_DEVINL void worker(const BsofGeom& g, const BsofState& st, double* sV, dou
     const int x2 = tile_id(g, m2, t2);
     const int rows = 2 * g.n - f.j0, nb = (rows + 7) / 8;
     long long ldp, ldc;
-    const double* P = mat_ptr(g, st, (long long)f.k * g.n + f.j0, f.m, f.t * 16, ldp);
+    const double* P = mat_ptr(g, st, (long long)f.k * g.n + f.j0, f.m, f.t * g.NB, ldp);
     double* C = tile_ptr(g, st, f.k, f.j0, m2, t2, ldc);
-    const int w2 = min(16, g.n - t2 * 16);
+    const int w2 = min(g.NB, g.n - t2 * g.NB);
     // The tile is loaded while the leaf is still being factored.
     if (tid == 0) sm.flag = wait_geq(st, st.cnt + x2, s - lo2) ? 1 : 0;
     bar_main<MT>();
     if (!sm.flag) return;
-    double c[NIW][2][2];
+    double c[NIW][CN][2];
     const bool vecc = pair_aligned(C, ldc);
 #pragma unroll
     for (int i = 0; i < NIW; i++) {
       const int b = warp + i * MW;
 #pragma unroll
-      for (int cs = 0; cs < 2; cs++) {
+      for (int cs = 0; cs < K::CN; cs++) {
         const int cc = gc + 8 * cs;
         const double2 v = ld_pair(C + cm(0, cc, ldc), 8 * b + 2 * t, rows, b < nb && cc < w2, vecc);
         c[i][cs][0] = v.x;
@@ -1092,71 +1279,71 @@ BSOFI_DEVINL void worker(const BsofGeom& g, const BsofState& st, double* sV, dou
     // V (unit lower trapezoidal) and T to shared memory.
     {
       const bool vec = pair_aligned(P, ldp) && (rows & 1) == 0;
-      if (K::BULK && vec && tid == 0 && rows > 16) {
+      if (K::BULK && vec && tid == 0 && rows > LW) {
         fence_proxy();
-        tc::mbar_arrive_expect_tx(&sm.bar, 8 * f.w * (rows - 16));
+        tc::mbar_arrive_expect_tx(&sm.bar, 8 * f.w * (rows - LW));
         for (int cc = 0; cc < f.w; cc++)
-          bulk_load(sV + sidx(16, cc, SV), P + cm(16, cc, ldp), rows - 16, &sm.bar);
+          bulk_load(sV + sidx(LW, cc, SV), P + cm(LW, cc, ldp), rows - LW, &sm.bar);
       }
       if (!vec) {
 #pragma unroll
-        for (int cc = warp; cc < 16; cc += 2 * MW)
-          copy_cols<2, K::LOADS>(sV, SV, P, ldp, cc, MW, f.w, 16, rows, lane);
+        for (int cc = warp; cc < LW; cc += 2 * MW)
+          copy_cols<2, K::LOADS>(sV, SV, P, ldp, cc, MW, f.w, LW, rows, lane);
       }
-      for (int cc = warp; cc < 16; cc += MW) {
+      for (int cc = warp; cc < LW; cc += MW) {
         const double* col = P + cm(0, cc, ldp);
         if (cc >= f.w) {
-          for (int r = 16 + lane; r < 8 * nb; r += 32) sV[sidx(r, cc, SV)] = 0.0;
+          for (int r = LW + lane; r < 8 * nb; r += 32) sV[sidx(r, cc, SV)] = 0.0;
         } else if (vec) {
           if (!K::BULK) {
 #pragma unroll 1
-            for (int r = 16 + 2 * lane; r < rows; r += 64)
+            for (int r = LW + 2 * lane; r < rows; r += 64)
               cp_async16(sV + sidx(r, cc, SV), col + r, 16);
           }
-          if (lane < 8 && max(rows, 16) + lane < 8 * nb) sV[sidx(max(rows, 16) + lane, cc, SV)] = 0.0;
-        } else if (lane < 8 && max(rows, 16) + lane < 8 * nb) {
-          sV[sidx(max(rows, 16) + lane, cc, SV)] = 0.0;
+          if (lane < 8 && max(rows, LW) + lane < 8 * nb) sV[sidx(max(rows, LW) + lane, cc, SV)] = 0.0;
+        } else if (lane < 8 && max(rows, LW) + lane < 8 * nb) {
+          sV[sidx(max(rows, LW) + lane, cc, SV)] = 0.0;
         }
       }
       const double* T = st.T + ((long long)f.k * st.maxleaves + f.l) * 256;
-      for (int e = tid; e < 256; e += MT) {
-        const int r = e & 15, cc = e >> 4;
+      for (int e = tid; e < LW * LW; e += MT) {
+        const int r = e % LW, cc = e / LW;
         double v = 0.0;
         if (cc < f.w && r < rows) v = r == cc ? 1.0 : (r > cc ? __ldcg(P + cm(r, cc, ldp)) : 0.0);
         sV[sidx(r, cc, SV)] = v;
-        sm.T[r][cc] = __ldcg(T + e);
+        sm.T[r][cc] = __ldcg(T + r + 16 * cc);
       }
       if (!K::BULK) {
         cp_async_wait<0>();
-      } else if (vec && rows > 16) {
+      } else if (vec && rows > LW) {
         if (tid == 0 && !bulk_wait(&sm.bar, phase, st.err)) sm.flag = 0;
         phase ^= 1;
       }
     }
     bar_main<MT>();
     if (!sm.flag) return;
-    double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+    double acc[CN][2 * CN] = {};
 #pragma unroll
     for (int i = 0; i < NIW; i++) {
       const int b = warp + i * MW;
       if (b < nb) {
 #pragma unroll
-        for (int jt = 0; jt < 2; jt++) {
+        for (int jt = 0; jt < CN; jt++) {
           const double2 v =
               *reinterpret_cast<const double2*>(sV + sidx(8 * b + 2 * t, gc + 8 * jt, SV));
-          dmma_16x8x8(acc[jt], c[i][0][0], c[i][1][0], c[i][0][1], c[i][1][1], v.x, v.y);
+          mma_w<CN>(acc[jt], c[i], v.x, v.y);
         }
       }
     }
-    double fr[2][4];
-    reduce_w<MW>(acc, fr, part, sm, gq, t, warp);
+    double fr[CN][2 * CN];
+    reduce_w<MW, CN>(acc, fr, part, sm, gq, t, warp);
 #pragma unroll
     for (int i = 0; i < NIW; i++) {
       const int b = warp + i * MW;
       if (b < nb) {
-        update_block(c[i], fr, sV, SV, 8 * b, gq, t);
+        update_block<CN>(c[i], fr, sV, SV, 8 * b, gq, t);
 #pragma unroll
-        for (int cs = 0; cs < 2; cs++)
+        for (int cs = 0; cs < K::CN; cs++)
           st_pair(C + cm(0, gc + 8 * cs, ldc), 8 * b + 2 * t, rows, gc + 8 * cs < w2, vecc,
                   c[i][cs][0], c[i][cs][1]);
       }
@@ -1169,21 +1356,230 @@ BSOFI_DEVINL void worker(const BsofGeom& g, const BsofState& st, double* sV, dou
   }
 }
 
+// Workers of the 8-wide forms.  A claimed task is a pair of neighbouring tiles
+// (16 columns) for a whole stage: its rows stay in registers while the stage's
+// leaves are applied one after another, so that a leaf costs the load of V and
+// the two products, and the tiles move twice a stage instead of twice a leaf.
+// Stage j is panel j's leaves; the final panel is two stages, the second one
+// (j = L-1) with its rows counted from row n of the panel.  Tiles of the stage
+// itself (block column j) need the leaves up to two before their own (the chain
+// applies the one before), the others all.  Tasks are claimed in order, a stage's own tiles
+// first and from the left: a task waits for leaves that depend on earlier
+// tasks only, so any number of workers ends.
+//
+// What bounds them: the tile of the leaf after next is due one chain step
+// (about 8 us) after a leaf is published, and all of a leaf's updates take
+// (3 nl/2 + nl with G) tasks of one V load (75 KB of L2) and 2 x 1.3 us of
+// DMMA at n = 576.  With one task per leaf and tile, as in worker(), an inversion
+// at n = 576, p = 12 took 21.5 ms, the chain waiting 8 of its 16 us a leaf
+// (each SM two or three tasks in a row, C in and out of L2 for each); so 18.7, and
+// 17.6 with the leaf published early.
+template <class K>
+BSOFI_DEVINL void holder(const BsofGeom& g, const BsofState& st, double* sV, double* part, int SV,
+                         ChainSmem<K::MW>& sm) {
+  constexpr int MW = K::MW, MT = K::MT, NIW = K::NIW, LW = K::LW;
+  static_assert(LW == 8, "a pair of 8-wide tiles is one 16-row operand");
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+  const int gq = lane >> 2, t = lane & 3, gc = col_of(gq);
+  const int n = g.n, L = g.L, nl = g.nl;
+  uint32_t phase = 0;
+  // Pairs per stage: its own tiles 1.., a block column, the halves of G.
+  const int own = nl / 2, half = (nl + 1) / 2, gp = g.form_g ? 2 * half : 0;
+  const int per = own + 2 * half + gp, regular = (L - 2) * per;
+  const int total = regular + (own + half + gp) + (own + gp);
+  for (;;) {
+    if (tid == 0) sm.task = atomicAdd(st.next_task, 1);
+    bar_main<MT>();
+    int q = sm.task;
+    if (q >= total) return;
+    int j = L - 2;
+    if (q < regular) {
+      j = q / per;
+      q -= j * per;
+    } else {
+      q -= regular;
+      if (q >= own + half + gp) {
+        q -= own + half + gp;
+        j = L - 1;
+      }
+    }
+    // Tiles t0, t0 + 1 of block column m, and how many of the stage's leaves each gets.
+    int m, t0, e0, e1;
+    if (q < own) {
+      m = j;
+      t0 = 1 + 2 * q;
+      e0 = t0 - 1;
+      e1 = t0;
+    } else {
+      q -= own;
+      const int part_of = q / half, nmat = j <= L - 3 ? 2 : (j == L - 2 ? 1 : 0);
+      t0 = 2 * (q % half);
+      m = part_of >= nmat ? L + 2 * min(j, L - 2) + part_of - nmat : (part_of == 0 ? j + 1 : L - 1);
+      // The chain applies a leaf to its first target: the stage's last leaf to tile 0 of block
+      // column j+1, and after the last one of all to the first tile of G.
+      const bool first = m == j + 1 || (j == L - 1 && m == L + 2 * (L - 2));
+      e0 = first && t0 == 0 ? nl - 1 : nl;
+      e1 = nl;
+    }
+    if (t0 + 1 >= nl) e1 = 0;
+    int lo, hi;
+    tile_range(g, m, t0, lo, hi);
+    int* cnt = st.cnt + tile_id(g, m, t0);
+    if (tid == 0)
+      sm.flag = (e0 == 0 || wait_geq(st, cnt, j * nl - lo)) &&
+                        (e1 == 0 || wait_geq(st, cnt + 1, j * nl - lo))
+                    ? 1
+                    : 0;
+    bar_main<MT>();
+    if (!sm.flag) return;
+    const int k = min(j, L - 2), base = j == L - 1 ? n : 0;
+    const int rows = 2 * n - base, nb = (rows + 7) / 8, w2 = min(2 * LW, n - t0 * LW);
+    long long ldc;
+    double* C = tile_ptr(g, st, k, base, m, t0, ldc);
+    const bool vecc = pair_aligned(C, ldc);
+    double c[NIW][2][2];
+#pragma unroll
+    for (int i = 0; i < NIW; i++) {
+      const int b = warp + i * MW;
+#pragma unroll
+      for (int cs = 0; cs < 2; cs++) {
+        const double2 v = ld_pair(C + cm(0, gc + 8 * cs, ldc), 8 * b + 2 * t, rows,
+                                  b < nb && gc + 8 * cs < w2 && (cs == 0 ? e0 : e1) > 0, vecc);
+        c[i][cs][0] = v.x;
+        c[i][cs][1] = v.y;
+      }
+    }
+#pragma unroll 1
+    for (int l = 0; l < max(e0, e1); l++) {
+      const int s = j * nl + l, ab = LW * l;
+      bar_main<MT>();  // everyone has read sm.flag and V
+      if (tid == 0) sm.flag = wait_geq(st, st.factored + s, 1) ? 1 : 0;
+      bar_main<MT>();
+      if (!sm.flag) return;
+      // V (unit lower trapezoidal) and T to shared memory.
+      {
+        const Leaf f = leaf_of(g, s);
+        long long ldp;
+        const double* P = mat_ptr(g, st, (long long)k * n + f.j0, f.m, f.t * LW, ldp);
+        const int left = rows - ab;  // rows from the leaf's first on
+        const bool vec = pair_aligned(P, ldp) && (left & 1) == 0;
+        double* V = sV + ab;
+        if (tid == 0 && left > LW) {
+          issue_columns(V + LW, SV, P + LW, ldp, f.w, left - LW, vec, &sm.bar);
+        }
+        static_assert(MW == LW, "a warp per column");
+        if (warp >= f.w) {
+          for (int r = LW + lane; r < 8 * nb - ab; r += 32) V[sidx(r, warp, SV)] = 0.0;
+        } else {
+          if (max(left, LW) + lane < 8 * nb - ab) V[sidx(max(left, LW) + lane, warp, SV)] = 0.0;
+        }
+        const double* T = st.T + ((long long)f.k * st.maxleaves + f.l) * 256;
+        if (tid < LW * LW) {
+          const int r = tid % LW, cc = tid / LW;
+          double v = 0.0;
+          if (cc < f.w && r < left) v = r == cc ? 1.0 : (r > cc ? __ldcg(P + cm(r, cc, ldp)) : 0.0);
+          V[sidx(r, cc, SV)] = v;
+        } else if (tid < 2 * LW * LW) {
+          const int r = tid % LW, cc = (tid - LW * LW) / LW;
+          sm.T[r][cc] = __ldcg(T + r + 16 * cc);
+        }
+        if (left > LW) {
+          if (tid == 0 && !bulk_wait(&sm.bar, phase, st.err)) sm.flag = 0;
+          phase ^= 1;
+          if (!vec) {
+            bar_main<MT>();
+            if (warp < f.w)
+              span_finish(V + sidx(LW, warp, SV), P + cm(LW, warp, ldp), left - LW, lane);
+          }
+        }
+      }
+      bar_main<MT>();
+      if (!sm.flag) return;
+      double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int i = 0; i < NIW; i++) {
+        const int b = warp + i * MW;
+        if (b < l || b >= nb) continue;
+        const double2 v = *reinterpret_cast<const double2*>(sV + sidx(8 * b + 2 * t, gc, SV));
+        dmma_16x8x8(acc, c[i][0][0], c[i][1][0], c[i][0][1], c[i][1][1], v.x, v.y);
+      }
+      // -(W^T T) summed over the warps, as in reduce_w.
+      double fr[4];
+      {
+        double o[4] = {0.0, 0.0, 0.0, 0.0};
+        dmma_16x8x8(o, acc[0], acc[2], acc[1], acc[3], sm.T[t][gq], sm.T[t + 4][gq]);
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+          *reinterpret_cast<double2*>(part + warp * 128 + (gc + 8 * h) * 8 + 2 * t) =
+              make_double2(o[2 * h], o[2 * h + 1]);
+        bar_main<MT>();
+        if (tid < 128) {
+          double sum[MW];
+#pragma unroll
+          for (int u = 0; u < MW; u++) sum[u] = part[u * 128 + tid];
+#pragma unroll
+          for (int d = MW / 2; d > 0; d /= 2)
+#pragma unroll
+            for (int u = 0; u < d; u++) sum[u] += sum[u + d];
+          sm.W[tid] = -sum[0];
+        }
+        bar_main<MT>();
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const double2 v = *reinterpret_cast<const double2*>(sm.W + (gc + 8 * h) * 8 + 2 * t);
+          fr[h] = v.x;
+          fr[2 + h] = v.y;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < NIW; i++) {
+        const int b = warp + i * MW;
+        if (b < l || b >= nb) continue;
+        double d[4] = {c[i][0][0], c[i][0][1], c[i][1][0], c[i][1][1]};
+        dmma_16x8x8(d, fr[0], fr[1], fr[2], fr[3], sV[sidx(8 * b + gq, 2 * t, SV)],
+                    sV[sidx(8 * b + gq, 2 * t + 1, SV)]);
+        c[i][0][0] = d[0];
+        c[i][0][1] = d[1];
+        c[i][1][0] = d[2];
+        c[i][1][1] = d[3];
+      }
+      const bool out0 = l + 1 == e0, out1 = l + 1 == e1;
+      if (out0 || out1) {
+#pragma unroll
+        for (int i = 0; i < NIW; i++) {
+          const int b = warp + i * MW;
+          if (b >= nb) continue;
+#pragma unroll
+          for (int cs = 0; cs < 2; cs++)
+            st_pair(C + cm(0, gc + 8 * cs, ldc), 8 * b + 2 * t, rows,
+                    gc + 8 * cs < w2 && (cs == 0 ? out0 : out1), vecc, c[i][cs][0], c[i][cs][1]);
+        }
+        bar_main<MT>();
+        if (tid == 0) {
+          __threadfence();
+          if (out0) red_release_add(cnt, e0);
+          if (out1) red_release_add(cnt + 1, e1);
+        }
+      }
+    }
+  }
+}
+
 template <class K>
 __global__ void __launch_bounds__(K::THREADS, 1) bsof_persistent_kernel(BsofGeom g, BsofState st) {
   extern __shared__ __align__(16) double dyn_bsof[];
   __shared__ __align__(16) ChainSmem<K::MW> sm;
   const int SV = tile_stride(g.n);
   double* sV = dyn_bsof;
-  double* part = sV + 16 * SV;
-  double* sC = part + K::MW * 256;
+  double* part = sV + K::LW * SV;
+  double* sC = part + K::MW * 16 * K::LW;
   if (threadIdx.x == 0) {
     tc::mbar_init(&sm.bar, 1);
     tc::fence_barrier_init();
   }
-  if (blockIdx.x == 0) {
-    if (threadIdx.x == 0) sm.step[st.s_begin & 1] = chain_step(g, st, st.s_begin);
-      }
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    sm.step[st.s_begin & 1] = chain_step(g, st, st.s_begin);
   __syncthreads();
   if (threadIdx.x >= K::MT) {
     if constexpr (K::REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
@@ -1191,6 +1587,7 @@ __global__ void __launch_bounds__(K::THREADS, 1) bsof_persistent_kernel(BsofGeom
   } else {
     if constexpr (K::REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
     if (blockIdx.x == 0) chain_main<K>(g, st, sV, part, sC, SV, sm);
+    else if constexpr (K::CN == 1) holder<K>(g, st, sV, part, SV, sm);
     else worker<K>(g, st, sV, part, SV, sm);
   }
 }
@@ -1277,11 +1674,11 @@ __global__ void __launch_bounds__(K::MT, PER) form_q_kernel(FormQArgs s) {
       }
     }
     double fr[2][4];
-    reduce_w<MW>(acc, fr, part, sm, gq, t, warp);
+    reduce_w<MW, 2>(acc, fr, part, sm, gq, t, warp);
 #pragma unroll
     for (int i = 0; i < NIW; i++) {
       const int b = warp + i * MW;
-      if (8 * b + 7 >= j0 && b < nb) update_block(c[i], fr, sV, SV, 8 * b, gq, t);
+      if (8 * b + 7 >= j0 && b < nb) update_block<2>(c[i], fr, sV, SV, 8 * b, gq, t);
     }
     bar_main<MT>();  // V, T and W are no longer read
   }
@@ -1301,10 +1698,13 @@ using Chain64 = ChainCfg<3, 5, 4>;
 using Chain128 = ChainCfg<7, 5, 4>;
 using Chain256 = ChainCfg<7, 9, 8>;
 using Chain400 = ChainCfg<7, 14, 13>;
-using Chain640 = ChainCfg<7, 23, 20>;  // (its worker shape only: form_q_kernel)
+using Chain592 = ChainCfg<7, 21, 19, 1>;
+using Chain640 = ChainCfg<7, 23, 20, 1>;
+using FormQ640 = ChainCfg<7, 23, 20>;
 
 // 16-wide leaves up to n = 400, where the next tile still fits in shared
-// memory beside V; the tall kernel's 8-wide ones above.
+// memory beside V (16-wide ones above, without it: n = 450, p = 3 5.7 ms against
+// 4.0 with 8-wide ones); 8-wide above.
 int bsof_leaf_width(int n) { return n <= Chain400::MAX_ROWS / 2 ? 16 : 8; }
 
 int bsof_tiles(int n) { return (n + bsof_leaf_width(n) - 1) / bsof_leaf_width(n); }
@@ -1312,7 +1712,7 @@ int bsof_tiles(int n) { return (n + bsof_leaf_width(n) - 1) / bsof_leaf_width(n)
 template <class K>
 static size_t dyn_smem(int n) {
   const size_t SV = tile_stride(n);
-  return sizeof(double) * (16 * SV + 256 * K::MW + 16 * (SV + 16));
+  return sizeof(double) * (K::LW * SV + 16 * K::LW * K::MW + K::LW * (SV + 16));
 }
 
 template <class K>
@@ -1373,6 +1773,9 @@ cudaError_t launch_bsof_persistent(double* A, long long ld, int n, int L, double
   if (2 * n <= Chain128::MAX_ROWS) return launch_cfg<Chain128>(g, s, workers, st);
   if (2 * n <= Chain256::MAX_ROWS) return launch_cfg<Chain256>(g, s, workers, st);
   if (2 * n <= Chain400::MAX_ROWS) return launch_cfg<Chain400>(g, s, workers, st);
+  if (s.s_begin > 0 || s.s_end < g.S) return cudaErrorInvalidValue;  // stages are not split
+  if (2 * n <= Chain592::MAX_ROWS) return launch_cfg<Chain592>(g, s, workers, st);
+  if (2 * n <= Chain640::MAX_ROWS) return launch_cfg<Chain640>(g, s, workers, st);
   return launch_bsof_tall(g, s, workers, st);
 }
 
@@ -1393,7 +1796,7 @@ static cudaError_t launch_form_q_cfg(const FormQArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-bool form_q_fits(int n) { return 2 * n <= Chain640::MAX_ROWS; }
+bool form_q_fits(int n) { return 2 * n <= FormQ640::MAX_ROWS; }
 
 cudaError_t launch_form_q(const double* A, long long ld, int n, int L, const double* T,
                           int maxleaves, int nbw, double* G, cudaStream_t st) {
@@ -1402,7 +1805,7 @@ cudaError_t launch_form_q(const double* A, long long ld, int n, int L, const dou
   if (2 * n <= Chain128::MAX_ROWS) return launch_form_q_cfg<Chain128, 2>(a, st);
   if (2 * n <= Chain256::MAX_ROWS) return launch_form_q_cfg<Chain256, 2>(a, st);
   if (2 * n <= Chain400::MAX_ROWS) return launch_form_q_cfg<Chain400, 1>(a, st);
-  if (2 * n <= Chain640::MAX_ROWS) return launch_form_q_cfg<Chain640, 1>(a, st);
+  if (2 * n <= FormQ640::MAX_ROWS) return launch_form_q_cfg<FormQ640, 1>(a, st);
   return cudaErrorInvalidValue;
 }
 
@@ -1416,7 +1819,9 @@ cudaError_t preload_bsof(size_t* local) {
   if ((e = preload_one(form_q_kernel<Chain128, 2>, local)) != cudaSuccess) return e;
   if ((e = preload_one(form_q_kernel<Chain256, 2>, local)) != cudaSuccess) return e;
   if ((e = preload_one(form_q_kernel<Chain400, 1>, local)) != cudaSuccess) return e;
-  if ((e = preload_one(form_q_kernel<Chain640, 1>, local)) != cudaSuccess) return e;
+  if ((e = preload_one(form_q_kernel<FormQ640, 1>, local)) != cudaSuccess) return e;
+  if ((e = preload_one(bsof_persistent_kernel<Chain592>, local)) != cudaSuccess) return e;
+  if ((e = preload_one(bsof_persistent_kernel<Chain640>, local)) != cudaSuccess) return e;
   return preload_bsof_tall(local);
 }
 

@@ -1,9 +1,7 @@
-// BSOF for the tallest panels (n above the 16-wide leaves' limit, up to 768):
-// the schedule of kernels_bsof.cu with 8-wide leaves, so that 1536 rows fit
-// the registers of one CTA (TR = 4, 5 or 6 rows of eight columns a thread).
-// 16-wide leaves of that height leave no room to stage the next tile and spill
-// (n = 576, p = 12: 15.7 against 16.0 ms, but slower below: an inversion at
-// n = 450, p = 3 took 5.7 against 4.0 ms), so they end at n = 400.
+// BSOF for the tallest panels (n = 641..768): the schedule of kernels_bsof.cu
+// with 8-wide leaves and one task per leaf and tile, 1536 rows in the registers
+// of one CTA (six rows of eight columns a thread).  The layout of kernels_bsof.cu
+// needs the pivot column beside the leaf in registers, which ends at n = 640.
 #include <climits>
 #include "bsof_sched.cuh"
 #include "bsofi_kernels.h"
@@ -14,6 +12,7 @@ namespace {
 constexpr int BT = 256;  // threads per CTA
 constexpr int BW = BT / 32;
 constexpr int NB = 8;   // leaf width
+constexpr int ROWS_PER = 6;  // rows a thread
 
 // Sum NB values per lane over a warp (transpose reduction): lane l ends with
 // the warp sum of value (l >> 2) & 7.
@@ -410,17 +409,12 @@ cudaError_t launch_tr(const BsofGeom& g, const BsofState& st, int workers, cudaS
 }  // namespace
 
 cudaError_t launch_bsof_tall(const BsofGeom& g, const BsofState& st, int workers, cudaStream_t s) {
-  if (2 * g.n <= 4 * BT) return launch_tr<4>(g, st, workers, s);
-  if (2 * g.n <= 5 * BT) return launch_tr<5>(g, st, workers, s);
-  if (2 * g.n <= 6 * BT) return launch_tr<6>(g, st, workers, s);
+  if (2 * g.n <= ROWS_PER * BT) return launch_tr<ROWS_PER>(g, st, workers, s);
   return cudaErrorInvalidValue;
 }
 
 cudaError_t preload_bsof_tall(size_t* local) {
-  cudaError_t e;
-  if ((e = preload_one(bsof_tall_kernel<4>, local)) != cudaSuccess) return e;
-  if ((e = preload_one(bsof_tall_kernel<5>, local)) != cudaSuccess) return e;
-  return preload_one(bsof_tall_kernel<6>, local);
+  return preload_one(bsof_tall_kernel<ROWS_PER>, local);
 }
 
 }  // namespace bsofi
