@@ -47,7 +47,7 @@
 // five-level shuffle sum of 16 values a thread, the tile through L2 and shared
 // memory between leaves, 8-wide leaves above n = 256): n = 64, p = 16 1.03 ->
 // 0.55; n = 100, p = 64 6.87 -> 4.63; n = 256, p = 32 10.6 -> 7.1; n = 400,
-// p = 64 41.2 -> 32.  Per 16-column leaf at n = 256: 9.5 us of column steps
+// p = 64 41.2 -> 28 (8-wide).  Per 16-column leaf at n = 256: 9.5 us of column steps
 // (about 1160 cycles each, half of them FP64 issue: DFMA takes 3 cycles a warp
 // instruction per scheduler), 1.2 us for each half of the next tile's update
 // (64 cycles per m16n8k8, two row warps per scheduler).
@@ -89,7 +89,7 @@ struct ChainCfg {
   // EARLY: a leaf is published when V is in shared memory, not when the next tile
   // is, so that the workers' answer may take a chain step longer.  Where the chain
   // waits for them, an inversion at n = 576, p = 12 went from 19.6 to 17.6 ms and at
-  // n = 529 from 20.3 to 18.0; up to n = 400 it does not wait, and the extra barrier
+  // n = 529 from 20.3 to 18.0; 16-wide leaves do not wait, and the extra barrier
   // costs (n = 256, p = 32 11.65 -> 11.82, n = 400, p = 16 12.9 -> 13.3).
   static constexpr bool EARLY = CN == 1;
   // With 12 warps a thread gets 168 registers at launch; the helper warpgroup
@@ -1356,24 +1356,25 @@ BSOFI_DEVINL void worker(const BsofGeom& g, const BsofState& st, double* sV, dou
   }
 }
 
-// Workers of the 8-wide forms.  A claimed task is a pair of neighbouring tiles
-// (16 columns) for a whole stage: its rows stay in registers while the stage's
-// leaves are applied one after another, so that a leaf costs the load of V and
-// the two products, and the tiles move twice a stage instead of twice a leaf.
+// Workers of the 8-wide forms.  A claimed task is a tile or a pair of neighbouring
+// tiles (16 columns) for a whole stage: its rows stay in registers while the
+// stage's leaves are applied one after another, so that a leaf costs the load of V
+// and the two products, and the tiles move twice a stage instead of twice a leaf.
 // Stage j is panel j's leaves; the final panel is two stages, the second one
 // (j = L-1) with its rows counted from row n of the panel.  Tiles of the stage
 // itself (block column j) need the leaves up to two before their own (the chain
-// applies the one before), the others all.  Tasks are claimed in order, a stage's own tiles
-// first and from the left: a task waits for leaves that depend on earlier
+// applies the one before), the others all.  Tasks are claimed in order, a stage's
+// own tiles first and from the left: a task waits for leaves that depend on earlier
 // tasks only, so any number of workers ends.
 //
-// What bounds them: the tile of the leaf after next is due one chain step
-// (about 8 us) after a leaf is published, and all of a leaf's updates take
-// (3 nl/2 + nl with G) tasks of one V load (75 KB of L2) and 2 x 1.3 us of
-// DMMA at n = 576.  With one task per leaf and tile, as in worker(), an inversion
-// at n = 576, p = 12 took 21.5 ms, the chain waiting 8 of its 16 us a leaf
-// (each SM two or three tasks in a row, C in and out of L2 for each); so 18.7, and
-// 17.6 with the leaf published early.
+// What bounds them: the round trip from a published leaf to the tile of the leaf
+// after next (store of V, its load, the products, store and load of the tile), which
+// has one chain step and a half before the chain waits.  So a stage's own tiles, which
+// the chain needs next, are taken one by one (m8n8k4, half the time for the products)
+// and the others, whose time is the load of V, in pairs.  An inversion at n = 576,
+// p = 12 took 21.5 ms with one task per leaf and tile as in worker(), 18.7 with held
+// pairs, 17.4 with early publication, 17.1 with single own tiles (at n = 400,
+// p = 64 93.1 -> 91.2).
 template <class K>
 BSOFI_DEVINL void holder(const BsofGeom& g, const BsofState& st, double* sV, double* part, int SV,
                          ChainSmem<K::MW>& sm) {
@@ -1385,7 +1386,7 @@ BSOFI_DEVINL void holder(const BsofGeom& g, const BsofState& st, double* sV, dou
   const int n = g.n, L = g.L, nl = g.nl;
   uint32_t phase = 0;
   // Pairs per stage: its own tiles 1.., a block column, the halves of G.
-  const int own = nl / 2, half = (nl + 1) / 2, gp = g.form_g ? 2 * half : 0;
+  const int own = nl - 1, half = (nl + 1) / 2, gp = g.form_g ? 2 * half : 0;
   const int per = own + 2 * half + gp, regular = (L - 2) * per;
   const int total = regular + (own + half + gp) + (own + gp);
   for (;;) {
@@ -1408,9 +1409,9 @@ BSOFI_DEVINL void holder(const BsofGeom& g, const BsofState& st, double* sV, dou
     int m, t0, e0, e1;
     if (q < own) {
       m = j;
-      t0 = 1 + 2 * q;
+      t0 = 1 + q;
       e0 = t0 - 1;
-      e1 = t0;
+      e1 = 0;
     } else {
       q -= own;
       const int part_of = q / half, nmat = j <= L - 3 ? 2 : (j == L - 2 ? 1 : 0);
@@ -1423,6 +1424,7 @@ BSOFI_DEVINL void holder(const BsofGeom& g, const BsofState& st, double* sV, dou
       e1 = nl;
     }
     if (t0 + 1 >= nl) e1 = 0;
+    const bool pair = e1 > 0;
     int lo, hi;
     tile_range(g, m, t0, lo, hi);
     int* cnt = st.cnt + tile_id(g, m, t0);
@@ -1497,12 +1499,26 @@ BSOFI_DEVINL void holder(const BsofGeom& g, const BsofState& st, double* sV, dou
       bar_main<MT>();
       if (!sm.flag) return;
       double acc[4] = {0.0, 0.0, 0.0, 0.0};
+      if (pair) {
 #pragma unroll
-      for (int i = 0; i < NIW; i++) {
-        const int b = warp + i * MW;
-        if (b < l || b >= nb) continue;
-        const double2 v = *reinterpret_cast<const double2*>(sV + sidx(8 * b + 2 * t, gc, SV));
-        dmma_16x8x8(acc, c[i][0][0], c[i][1][0], c[i][0][1], c[i][1][1], v.x, v.y);
+        for (int i = 0; i < NIW; i++) {
+          const int b = warp + i * MW;
+          if (b < l || b >= nb) continue;
+          const double2 v = *reinterpret_cast<const double2*>(sV + sidx(8 * b + 2 * t, gc, SV));
+          dmma_16x8x8(acc, c[i][0][0], c[i][1][0], c[i][0][1], c[i][1][1], v.x, v.y);
+        }
+      } else {
+        double a2[2] = {0.0, 0.0};
+#pragma unroll
+        for (int i = 0; i < NIW; i++) {
+          const int b = warp + i * MW;
+          if (b < l || b >= nb) continue;
+          const double2 v = *reinterpret_cast<const double2*>(sV + sidx(8 * b + 2 * t, gc, SV));
+          dmma_8x8x4(a2, c[i][0][0], v.x);
+          dmma_8x8x4(a2, c[i][0][1], v.y);
+        }
+        acc[0] = a2[0];
+        acc[1] = a2[1];
       }
       // -(W^T T) summed over the warps, as in reduce_w.
       double fr[4];
@@ -1532,17 +1548,27 @@ BSOFI_DEVINL void holder(const BsofGeom& g, const BsofState& st, double* sV, dou
           fr[2 + h] = v.y;
         }
       }
+      if (pair) {
 #pragma unroll
-      for (int i = 0; i < NIW; i++) {
-        const int b = warp + i * MW;
-        if (b < l || b >= nb) continue;
-        double d[4] = {c[i][0][0], c[i][0][1], c[i][1][0], c[i][1][1]};
-        dmma_16x8x8(d, fr[0], fr[1], fr[2], fr[3], sV[sidx(8 * b + gq, 2 * t, SV)],
-                    sV[sidx(8 * b + gq, 2 * t + 1, SV)]);
-        c[i][0][0] = d[0];
-        c[i][0][1] = d[1];
-        c[i][1][0] = d[2];
-        c[i][1][1] = d[3];
+        for (int i = 0; i < NIW; i++) {
+          const int b = warp + i * MW;
+          if (b < l || b >= nb) continue;
+          double d[4] = {c[i][0][0], c[i][0][1], c[i][1][0], c[i][1][1]};
+          dmma_16x8x8(d, fr[0], fr[1], fr[2], fr[3], sV[sidx(8 * b + gq, 2 * t, SV)],
+                      sV[sidx(8 * b + gq, 2 * t + 1, SV)]);
+          c[i][0][0] = d[0];
+          c[i][0][1] = d[1];
+          c[i][1][0] = d[2];
+          c[i][1][1] = d[3];
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < NIW; i++) {
+          const int b = warp + i * MW;
+          if (b < l || b >= nb) continue;
+          dmma_8x8x4(c[i][0], fr[0], sV[sidx(8 * b + gq, 2 * t, SV)]);
+          dmma_8x8x4(c[i][0], fr[2], sV[sidx(8 * b + gq, 2 * t + 1, SV)]);
+        }
       }
       const bool out0 = l + 1 == e0, out1 = l + 1 == e1;
       if (out0 || out1) {
@@ -1697,15 +1723,19 @@ __global__ void __launch_bounds__(K::MT, PER) form_q_kernel(FormQArgs s) {
 using Chain64 = ChainCfg<3, 5, 4>;
 using Chain128 = ChainCfg<7, 5, 4>;
 using Chain256 = ChainCfg<7, 9, 8>;
-using Chain400 = ChainCfg<7, 14, 13>;
+using Chain416 = ChainCfg<7, 15, 13, 1>;
+using FormQ400 = ChainCfg<7, 14, 13>;
 using Chain592 = ChainCfg<7, 21, 19, 1>;
 using Chain640 = ChainCfg<7, 23, 20, 1>;
 using FormQ640 = ChainCfg<7, 23, 20>;
 
-// 16-wide leaves up to n = 400, where the next tile still fits in shared
-// memory beside V (16-wide ones above, without it: n = 450, p = 3 5.7 ms against
-// 4.0 with 8-wide ones); 8-wide above.
-int bsof_leaf_width(int n) { return n <= Chain400::MAX_ROWS / 2 ? 16 : 8; }
+// Leaf width.  Wide leaves halve the publications and updates, but a column step's
+// two column sets and an update's 16 columns cost the chain more than twice the
+// narrow ones' time once a warp has many row blocks: inversion in ms, 16-wide ->
+// 8-wide with held tiles: n = 300, p = 20 11.7 -> 10.3; 361, 20 17.1 -> 16.2; 400, 64
+// 95.6 -> 91.2.  Up to n = 256 the 16-wide leaves' chain does not wait for its
+// workers, and their fine tasks suit the few workers of a batch's instances.
+int bsof_leaf_width(int n) { return n <= Chain256::MAX_ROWS / 2 ? 16 : 8; }
 
 int bsof_tiles(int n) { return (n + bsof_leaf_width(n) - 1) / bsof_leaf_width(n); }
 
@@ -1772,8 +1802,8 @@ cudaError_t launch_bsof_persistent(double* A, long long ld, int n, int L, double
   if (2 * n <= Chain64::MAX_ROWS) return launch_cfg<Chain64>(g, s, workers, st);
   if (2 * n <= Chain128::MAX_ROWS) return launch_cfg<Chain128>(g, s, workers, st);
   if (2 * n <= Chain256::MAX_ROWS) return launch_cfg<Chain256>(g, s, workers, st);
-  if (2 * n <= Chain400::MAX_ROWS) return launch_cfg<Chain400>(g, s, workers, st);
   if (s.s_begin > 0 || s.s_end < g.S) return cudaErrorInvalidValue;  // stages are not split
+  if (2 * n <= Chain416::MAX_ROWS) return launch_cfg<Chain416>(g, s, workers, st);
   if (2 * n <= Chain592::MAX_ROWS) return launch_cfg<Chain592>(g, s, workers, st);
   if (2 * n <= Chain640::MAX_ROWS) return launch_cfg<Chain640>(g, s, workers, st);
   return launch_bsof_tall(g, s, workers, st);
@@ -1804,7 +1834,7 @@ cudaError_t launch_form_q(const double* A, long long ld, int n, int L, const dou
   if (2 * n <= Chain64::MAX_ROWS) return launch_form_q_cfg<Chain64, 4>(a, st);
   if (2 * n <= Chain128::MAX_ROWS) return launch_form_q_cfg<Chain128, 2>(a, st);
   if (2 * n <= Chain256::MAX_ROWS) return launch_form_q_cfg<Chain256, 2>(a, st);
-  if (2 * n <= Chain400::MAX_ROWS) return launch_form_q_cfg<Chain400, 1>(a, st);
+  if (2 * n <= FormQ400::MAX_ROWS) return launch_form_q_cfg<FormQ400, 1>(a, st);
   if (2 * n <= FormQ640::MAX_ROWS) return launch_form_q_cfg<FormQ640, 1>(a, st);
   return cudaErrorInvalidValue;
 }
@@ -1814,11 +1844,11 @@ cudaError_t preload_bsof(size_t* local) {
   if ((e = preload_one(bsof_persistent_kernel<Chain64>, local)) != cudaSuccess) return e;
   if ((e = preload_one(bsof_persistent_kernel<Chain128>, local)) != cudaSuccess) return e;
   if ((e = preload_one(bsof_persistent_kernel<Chain256>, local)) != cudaSuccess) return e;
-  if ((e = preload_one(bsof_persistent_kernel<Chain400>, local)) != cudaSuccess) return e;
+  if ((e = preload_one(bsof_persistent_kernel<Chain416>, local)) != cudaSuccess) return e;
   if ((e = preload_one(form_q_kernel<Chain64, 4>, local)) != cudaSuccess) return e;
   if ((e = preload_one(form_q_kernel<Chain128, 2>, local)) != cudaSuccess) return e;
   if ((e = preload_one(form_q_kernel<Chain256, 2>, local)) != cudaSuccess) return e;
-  if ((e = preload_one(form_q_kernel<Chain400, 1>, local)) != cudaSuccess) return e;
+  if ((e = preload_one(form_q_kernel<FormQ400, 1>, local)) != cudaSuccess) return e;
   if ((e = preload_one(form_q_kernel<FormQ640, 1>, local)) != cudaSuccess) return e;
   if ((e = preload_one(bsof_persistent_kernel<Chain592>, local)) != cudaSuccess) return e;
   if ((e = preload_one(bsof_persistent_kernel<Chain640>, local)) != cudaSuccess) return e;

@@ -25,7 +25,7 @@ from .hubbard import hubbard_blocks, hubbard_matrix, random_pcyclic
 
 
 def bsof_leaves(n, L):
-    nb = 16 if n <= 400 else 8
+    nb = 16 if n <= 256 else 8
     nl = (n + nb - 1) // nb
     return (L - 2) * nl + 2 * nl
 
@@ -72,7 +72,7 @@ def bsof_timeline(n, L, reps=3):
             "to_next_leaf_us": (t[1:, 0] - t[:-1, 2]).mean() / 1e3,
         }
         wait = (t[:, 1] - t[:, 0]) / 1e3
-        nl = (n + (16 if n <= 400 else 8) - 1) // (16 if n <= 400 else 8)
+        nl = (n + (16 if n <= 256 else 8) - 1) // (16 if n <= 256 else 8)
         first = np.arange(S) % nl == 0  # the first leaf of each regular panel
         first[(L - 2) * nl:] = False
         out.update({

@@ -18,12 +18,12 @@ from conftest import inverse_tolerance, rel_fro, split_state
 
 pytestmark = pytest.mark.gpu
 
-# (n, L): 64 / 128 / 256 / 400 / 592 / 640 are the largest blocks of the kernel's
-# forms; leaves of 16 (8 above 400) columns end evenly, one short and one over;
+# (n, L): 64 / 128 / 256 / 416 / 592 / 640 are the largest blocks of the kernel's
+# forms; leaves of 16 (8 above 256) columns end evenly, one short and one over;
 # odd n with an odd number of blocks has columns of both alignments.
 SIZES = [(1, 2), (15, 3), (16, 2), (17, 5), (32, 3), (63, 3), (64, 4), (65, 3), (127, 2), (128, 3),
-         (129, 2), (129, 3), (136, 3), (255, 2), (256, 2), (257, 2), (392, 2), (400, 2), (401, 2), (401, 3), (592, 2),
-         (593, 3), (640, 2), (641, 2)]
+         (129, 2), (129, 3), (136, 3), (255, 2), (256, 2), (257, 2), (257, 3), (392, 2), (400, 2),
+         (401, 2), (401, 3), (416, 2), (417, 2), (592, 2), (593, 3), (640, 2), (641, 2)]
 
 
 @pytest.mark.parametrize("n,L", SIZES)
