@@ -4,8 +4,8 @@
 // the stacked 2n x n panel [R~_k; B_k] at A_BLK(k,k), dormqr('L','T') of
 // A_BLK(k,k+1) and A_BLK(k,L-1); then dgeqrf of the final 2n x 2n block.
 //
-// Work decomposition.  Every block column is cut into tiles of 16 columns
-// (the last one may be narrower).  A "leaf" is the Householder QR of one tile
+// Work decomposition.  Every block column is cut into tiles of 16 columns, 8
+// above n = 256 (the last one may be narrower).  A "leaf" is the Householder QR of one tile
 // inside its panel; leaves are numbered s = 0..S-1 in the reference's order
 // (panel k, left to right; the final panel has the tiles of block columns L-2
 // and L-1).  Leaf s updates a set of target tiles with its block reflector
@@ -27,7 +27,7 @@
 // The chain is a serial sequence of N Householder columns, so its time is the
 // latency of one column step.  The leaf stays in registers from one leaf to
 // the next, laid out as the accumulators of mma.m16n8k8.f64 hold C^T: lane
-// 4 g + t of a warp owns two columns and rows 2t, 2t+1 of each of its 8-row
+// 4 g + t of a warp owns two columns (one of an 8-wide leaf) and rows 2t, 2t+1 of each of its 8-row
 // blocks.  That layout makes a column step cheap in every part: the pivot
 // column reaches the lanes of a row block by one shuffle per row, a column's
 // dot products end in a sum over four lanes (a DMMA with ones), and there is
@@ -36,7 +36,7 @@
 // forming them for all, measured the same at n = 256 and slower below; two
 // columns per barrier, the second one's products corrected for the first
 // reflector, measured slower everywhere: one warp's scalar code then takes
-// longer than the barrier it saves).  The 16 pivot rows of a leaf belong to
+// longer than the barrier it saves).  The pivot rows of a leaf belong to
 // one warp of their own (the top warp), so the row warps need no row masks; T
 // is built one column behind by another.  The same registers are the B operand
 // of W^T = C^T V and the accumulators of C^T -= (W T)^T V^T, so the update of
@@ -47,7 +47,7 @@
 // five-level shuffle sum of 16 values a thread, the tile through L2 and shared
 // memory between leaves, 8-wide leaves above n = 256): n = 64, p = 16 1.03 ->
 // 0.55; n = 100, p = 64 6.87 -> 4.63; n = 256, p = 32 10.6 -> 7.1; n = 400,
-// p = 64 41.2 -> 28 (8-wide).  Per 16-column leaf at n = 256: 9.5 us of column steps
+// p = 64 41.2 -> 28, n = 576, p = 12 16.0 -> 9.7 (8-wide).  Per 16-column leaf at n = 256: 9.5 us of column steps
 // (about 1160 cycles each, half of them FP64 issue: DFMA takes 3 cycles a warp
 // instruction per scheduler), 1.2 us for each half of the next tile's update
 // (64 cycles per m16n8k8, two row warps per scheduler).
