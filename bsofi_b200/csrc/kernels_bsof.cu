@@ -1329,6 +1329,7 @@ BSOFI_DEVINL void worker(const BsofGeom& g, const BsofState& st, double* sV, dou
         sm.T[r][cc] = __ldcg(T + r + 16 * cc);
       }
       if (!K::BULK) {
+        cp_async_commit();
         cp_async_wait<0>();
       } else if (vec && rows > LW) {
         if (tid == 0 && !bulk_wait(&sm.bar, phase, st.err)) sm.flag = 0;
