@@ -144,9 +144,19 @@ static int batch_workers(int n, int in_flight) {
   return n >= 180 || in_flight < 6 ? 16 : 96 / in_flight;
 }
 
-/* The same settings for the server's requests (server.c). */
+/* The same switches for the server's requests (server.c). */
 int bsofi_batch_pipelined_now(void) { return flag_get(&g_pipelined); }
-int bsofi_batch_workers_for(int n) { return batch_workers(n, MAX_STREAMS); }
+/* Workers of a request.  The server does not know what will be beside it, and a
+ * request alone waits for its chain, which starves from n = 224 on with fewer
+ * than 12: one request after the other, sides 15..16, 251 ms a run of 16 with the
+ * kernels and the 12 workers of before, 247 with 12, 280 with 10.  Below, 10 against
+ * the 6 of before: slots 2 / 4 / 8, sides 8..16, 95 / 82 / 122 ms a run with 6, 75 /
+ * 74 / 119 with 10 (and 12 from n = 224 on). */
+int bsofi_batch_workers_for(int n) {
+  const int w = flag_get(&g_batch_workers);
+  if (w > 0) return w;
+  return n > 256 ? 24 : (n >= 224 ? 12 : 10);
+}
 
 unsigned long long bsofi_batch_workspace_bytes_ex(int count, const int *n, const int *L,
                                                   const int *ldda, int precision) {
