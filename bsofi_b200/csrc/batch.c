@@ -123,24 +123,34 @@ void bsofi_device_set_batch_chains(int k) {
 static int g_pipelined = 1;
 void bsofi_device_set_batch_pipelined(int on) { flag_set(&g_pipelined, on ? 1 : 0); }
 
-/* BSOF worker CTAs per instance of a batch (0: by block size and the number of
- * instances in flight).  A chain's workers hold their SMs while it runs, so
- * the best count falls as more chains run together; with few chains the large
- * blocks end last and take more.  Measured on pipelined batches of mixed sizes
- * (n = 64..256, p = 8..64; ms a batch with 6 workers below n = 224 and 12 from
- * there on -> with this rule): 48 instances 230.6 -> 223.7, 20 90.5 -> 87.3,
- * 16 67.9 -> 67.2, 14 96.8 -> 94.4, 12 40.9 -> 41.2 and 32.3 -> 31.2, 9
+/* BSOF workers per instance of a batch (0: by block size, instances and streams).
+ * A launch that forms every Q_k^T, as these do, has two CTAs a worker and one for
+ * the chain, each filling its SM, and eight a worker above n = 256, at most the
+ * GPU's.  They hold their SMs while the chain runs, so the best count falls as more
+ * chains run together.  Measured on pipelined batches of mixed sizes (n = 64..256,
+ * p = 8..64, one stream an instance; ms a batch with 6 workers below n = 224 and 12
+ * from there on -> with this rule): 48 instances on 16 streams 230.6 -> 223.7, 20
+ * 90.5 -> 87.3, 16 67.9 -> 67.2, 14 96.8 -> 94.4, 12 40.9 -> 41.2 and 32.3 -> 31.2, 9
  * 48.6 -> 34.6, 7 30.0 -> 18.5, 4 44.0 -> 32.4.  The line at 12 in flight: 13 and
  * 16 instances took 79.8 and 67.1 with 10 for all, 85.1 and 70.6 with 14 and 12
  * for the large ones; 12 instances 36.8 with 10 for all, 31.2 with 16 and 8.
- * Panels of n > 256 take 24. */
+ * Where instances queue behind 6 to 12 streams the GPU is full of their products
+ * and the few chains' 25 to 33 CTAs keep SMs from them: 8, and 12 for the large
+ * blocks.  On 8 streams, with 12 and 16 -> 8 and 12: 48 instances 138.3 -> 133.8, 20
+ * 56.0 -> 53.7, 17 48.8 -> 45.8, 14 36.3 -> 34.4, 12 of n <= 121 20.8 -> 17.7, 12 of
+ * all sizes 55.9 -> 54.4 and (a single large one at the end) 25.3 -> 32.7.  Four
+ * chains of 33 CTAs fit the GPU, so 4 and 5 streams do so only where the queue is
+ * deep: 48 instances on 4 streams 143.8 -> 138.1, 36 150.4 -> 150.2, but 20
+ * 37.4 with 16, 39.9 with 8 and 12. */
 static int g_batch_workers = 0;
 void bsofi_device_set_batch_workers(int w) { flag_set(&g_batch_workers, w < 0 ? 0 : w); }
-static int batch_workers(int n, int in_flight) {
+int bsofi_batch_workers(int n, int count, int in_flight) {
   const int w = flag_get(&g_batch_workers);
   if (w > 0) return w;
   if (n > 256) return 24;
   if (in_flight > 12) return 10;
+  if (in_flight >= 6 ? count > in_flight : in_flight >= 4 && count > 8 * in_flight)
+    return n >= 224 ? 12 : 8;
   return n >= 180 || in_flight < 6 ? 16 : 96 / in_flight;
 }
 
@@ -216,7 +226,7 @@ static int grouped_fp64(stream_pool *p, int used, int count, const int *n, const
   }
   for (i = 0; i < count && !r; i++) {
     const int k = ord[i].i;
-    const int workers = batch_workers(n[k], used);
+    const int workers = bsofi_batch_workers(n[k], count, used);
     r = bsofi_dev_bsoftri_q_ex(n[k], L[k], dA[k], ldda[k], dtau[k], ws[k], p->s[i % used],
                                workers);
     *launches += bsofi_dev_launch_count();
@@ -306,7 +316,7 @@ int bsofi_device_invert_batched_ex(int count, const int *n, const int *L, double
     bsofi_dev_set_nonpersistent(1);
     for (i = 0; i < count && !r; i++) {
       const int k = ord[i].i, slot = i % used;
-      const int workers = batch_workers(n[k], used);
+      const int workers = bsofi_batch_workers(n[k], count, used);
       r = bsofi_dev_invert_two_streams(n[k], L[k], dA[k], ldda[k], dtau[k],
                                        (char *)dwork + off[k], p->hi[slot], p->s[slot],
                                        p->gate[slot], workers,
@@ -322,7 +332,7 @@ int bsofi_device_invert_batched_ex(int count, const int *n, const int *L, double
   for (i = 0; i < count && !(precision == 0 && grouped) && !pipelined; i++) {
     const int k = ord[i].i;
     /* Few BSOF workers per instance: the batch supplies the parallelism. */
-    const int workers = batch_workers(n[k], used);
+    const int workers = bsofi_batch_workers(n[k], count, used);
     /* Gate: instance i waits for the chain of instance i - K (ring slot
      * i % K, recorded by that instance after its BSOF) and records the slot
      * after its own; the host issues them in that order. */

@@ -1,4 +1,4 @@
-"""BSOF worker counts of the server's requests: host rule, no GPU."""
+"""BSOF worker counts of batches and of the server's requests: host rules, no GPU."""
 import pytest
 
 from bsofi_b200 import _lib
@@ -11,10 +11,31 @@ def test_server_request(n, workers):
     assert _lib.load().bsofi_batch_workers_for(n) == workers
 
 
+@pytest.mark.parametrize("count,streams", [(9, 8), (12, 8), (17, 8), (48, 8), (7, 6), (13, 12),
+                                           (48, 4), (41, 5)])
+def test_batch_behind_few_streams(count, streams):
+    """Instances that queue fill the GPU with their products: few workers for the chains."""
+    lib = _lib.load()
+    assert [lib.bsofi_batch_workers(n, count, streams) for n in (64, 223, 224, 256, 257)] == \
+        [8, 8, 12, 12, 24]
+
+
+@pytest.mark.parametrize("count,streams,small,large", [(1, 1, 16, 16), (5, 5, 16, 16), (6, 6, 16, 16),
+                                                       (8, 8, 12, 16), (12, 12, 8, 16),
+                                                       (13, 13, 10, 10), (48, 16, 10, 10),
+                                                       (20, 4, 16, 16), (32, 4, 16, 16),
+                                                       (40, 2, 16, 16)])
+def test_batch_one_stream_an_instance_or_room_for_all(count, streams, small, large):
+    lib = _lib.load()
+    assert [lib.bsofi_batch_workers(n, count, streams) for n in (64, 179, 180, 256, 257)] == \
+        [small, small, large, large, 24]
+
+
 def test_setting_wins():
     lib = _lib.load()
     lib.bsofi_device_set_batch_workers(5)
     try:
         assert [lib.bsofi_batch_workers_for(n) for n in (64, 256, 400)] == [5, 5, 5]
+        assert lib.bsofi_batch_workers(400, 48, 8) == 5
     finally:
         lib.bsofi_device_set_batch_workers(0)
