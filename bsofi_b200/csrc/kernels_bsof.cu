@@ -1725,12 +1725,13 @@ __global__ void __launch_bounds__(K::MT, PER) form_q_kernel(FormQArgs s) {
     bar_main<MT>();  // V, T and W are no longer read
   }
   double* C = s.G + (long long)k * n2 * n2 + cm(0, x0, n2);
+  const bool vecc = pair_aligned(C, n2);  // (as the caller's workspace is)
 #pragma unroll
   for (int i = 0; i < NIW; i++) {
     const int b = warp + i * MW;
 #pragma unroll
     for (int cs = 0; cs < 2; cs++)
-      st_pair(C + cm(0, gc + 8 * cs, n2), 8 * b + 2 * t, n2, b < nb && x0 + gc + 8 * cs < n2, true,
+      st_pair(C + cm(0, gc + 8 * cs, n2), 8 * b + 2 * t, n2, b < nb && x0 + gc + 8 * cs < n2, vecc,
               c[i][cs][0], c[i][cs][1]);
   }
 }
