@@ -1154,6 +1154,14 @@ int bsofi_selftest_gemm(int M, int N, int K, double alpha, const double *dA, int
   return e ? cuda_info((cudaError_t)e) : 0;
 }
 
+int bsofi_selftest_reflector(int count, const double *dxnorm2, const double *dalpha, double *dout,
+                             void *stream) {
+  int e;
+  if (count < 1 || !dxnorm2 || !dalpha || !dout) return -1;
+  e = bsofi_dev_selftest_reflector(count, dxnorm2, dalpha, dout, stream);
+  return e ? cuda_info((cudaError_t)e) : 0;
+}
+
 void bsofi_device_timing(int on) { bsofi_dev_timing(on); }
 
 int bsofi_device_timing_read(double *ms, long long *launches) {

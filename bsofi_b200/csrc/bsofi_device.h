@@ -221,6 +221,10 @@ void bsofi_dev_set_bstri_overlap(int on);
 int bsofi_dev_selftest_gemm(int M, int N, int K, double alpha, const double *dA, int lda,
                             int upper_a, const double *dB, int ldb, int upper_b, double beta,
                             double *dC, int ldc, int tile, void *stream);
+/* The BSOF chain's reflector scalars of `count` pairs (xnorm2, alpha), for
+ * tests: 7 doubles each (see bsofi_selftest_reflector). */
+int bsofi_dev_selftest_reflector(int count, const double *dxnorm2, const double *dalpha,
+                                 double *dout, void *stream);
 
 #ifdef __cplusplus
 }

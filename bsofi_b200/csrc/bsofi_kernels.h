@@ -59,6 +59,10 @@ cudaError_t launch_bsof_persistent(double* A, long long ld, int n, int L, double
                                    int workers, cudaStream_t st, int s_begin = 0,
                                    int s_end = -1, double* Al = nullptr, long long ldl = 0);
 
+// The chain's reflector scalars of `count` pairs (diagnostics): 7 doubles each.
+cudaError_t launch_reflector(int count, const double* xnorm2, const double* alpha, double* out,
+                             cudaStream_t st);
+
 // G_k = Q_k^T of every panel from the reflectors below A's panel diagonals and
 // the compact-WY factors T of leaves of nbw columns (kernels_bsof.cu).  Only
 // where form_q_fits.

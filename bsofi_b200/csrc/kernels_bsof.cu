@@ -373,12 +373,16 @@ struct Refl {
 // reciprocal and 1/(|alpha| + ||.||) are the longest dependent chain of a
 // column step, so they share one: Goldschmidt's coupled iteration (Markstein,
 // "Software division and square root using Goldschmidt's algorithms", 2004)
-// from the hardware's approximation gives norm and half its reciprocal
-// together, Newton's residual step finishes each, and the last reciprocal
-// starts from the first norm estimate meanwhile.  Against long double on 10^6
-// random pairs the largest errors are, in units of 2^-53, beta 1.48, tau 1.40, scale
-// 2.62 (with rsqrt() and a division: beta 1.92, scale 3.04).  Outside the range
-// where the approximations are normal numbers those functions are called.
+// from the hardware's approximation gives the norm and half its reciprocal
+// together, and a Newton step on the residual finishes each.  The last reciprocal
+// starts from the first norm estimate meanwhile and takes one step of
+// Chebyshev's third-order iteration (Traub, "Iterative Methods for the Solution
+// of Equations", 1964): with d = 1 - x z the reciprocal is z / (1 - d), of
+// whose series z (1 + d + d^2) keeps the terms that count at d of 2^-20.
+// Error bounds, counting a rounding as at most 2^-53: beta 1.5 units of it (half
+// of the sum's, one of the last step), q 2.5, tau 2.25, scale 3.5 and d^3.  The
+// self-test below samples them against long double.  Outside the range
+// where the approximations are normal numbers rsqrt() and a division are used.
 BSOFI_DEVINL Refl reflector(double xnorm2, double alpha) {
   Refl r;
   const double s2 = fma(alpha, alpha, xnorm2), aa = fabs(alpha);
@@ -418,6 +422,26 @@ BSOFI_DEVINL Refl reflector(double xnorm2, double alpha) {
     }
   }
   return r;
+}
+
+// Self-test: a warp per pair, whose lanes hold the same values as in a column
+// step; beta, tau, scale, q, and the first three by rsqrt() and a division.
+__global__ void __launch_bounds__(256) reflector_kernel(int count, const double* xnorm2,
+                                                        const double* alpha, double* out) {
+  const int i = (int)((blockIdx.x * 256ll + threadIdx.x) >> 5);
+  if (i >= count) return;
+  const double x2 = xnorm2[i], a = alpha[i];
+  const Refl r = reflector(x2, a);
+  if ((threadIdx.x & 31) != 0) return;
+  const double rs = rsqrt(fma(a, a, x2)), beta = -copysign(fma(a, a, x2) * rs, a);
+  double* o = out + 7ll * i;
+  o[0] = r.beta;
+  o[1] = r.tau;
+  o[2] = r.scale;
+  o[3] = r.q;
+  o[4] = beta;
+  o[5] = fma(fabs(a), rs, 1.0);
+  o[6] = 1.0 / (a - beta);
 }
 
 // Sum over the four lanes t of a column's group (lane 4 g + t), to all four:
@@ -1854,6 +1878,12 @@ cudaError_t launch_form_q(const double* A, long long ld, int n, int L, const dou
   if (2 * n <= FormQ400::MAX_ROWS) return launch_form_q_cfg<FormQ400, 1>(a, st);
   if (2 * n <= FormQ640::MAX_ROWS) return launch_form_q_cfg<FormQ640, 1>(a, st);
   return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_reflector(int count, const double* xnorm2, const double* alpha, double* out,
+                             cudaStream_t st) {
+  reflector_kernel<<<(unsigned)((count + 7ll) / 8), 256, 0, st>>>(count, xnorm2, alpha, out);
+  return cudaGetLastError();
 }
 
 cudaError_t preload_bsof(size_t* local) {

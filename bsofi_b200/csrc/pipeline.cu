@@ -1493,6 +1493,13 @@ int bsofi_dev_selftest_gemm(int M, int N, int K, double alpha, const double* dA,
   return 0;
 }
 
+int bsofi_dev_selftest_reflector(int count, const double* dxnorm2, const double* dalpha,
+                                 double* dout, void* stream) {
+  g_launches = 0;
+  CK(launch_reflector(count, dxnorm2, dalpha, dout, (cudaStream_t)stream));
+  return 0;
+}
+
 long long bsofi_dev_launch_count(void) { return g_launches; }
 
 void bsofi_dev_add_launches(long long c) { g_launches += c; }

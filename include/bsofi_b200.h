@@ -522,6 +522,15 @@ int bsofi_selftest_gemm(int M, int N, int K, double alpha, const double *dA, int
                         int upper_a, const double *dB, int ldb, int upper_b, double beta,
                         double *dC, int ldc, int tile, void *stream);
 
+/* Diagnostic entry point (no reference counterpart): the reflector scalars of
+ * the BSOF chain (dlarfg's beta, tau and 1/(alpha - beta), and -1/beta) of
+ * `count` pairs: the squared norm below the pivot and the pivot, device memory.
+ * dout: 7 doubles a pair, the four and then the first three as rsqrt() and a
+ * division give them.  Enqueued on `stream`; returns 0, -1 for an illegal
+ * argument or BSOFI_INFO_CUDA - error. */
+int bsofi_selftest_reflector(int count, const double *dxnorm2, const double *dalpha, double *dout,
+                             void *stream);
+
 /* Diagnostic entry point (no reference counterpart): one product C = A B
  * (column-major, M x K times K x N, K <= 1536) on the int8 tensor cores by the
  * Ozaki scheme with `slices` slices (0 = 8), as the mixed-precision BSOI
