@@ -997,8 +997,9 @@ BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const dou
       }
     }
     bar_ready<K::THREADS>();
-    if (ht == 0) st.timeline[4 * s + 3] = gtimer();
     const bool go = ok != 0;
+    // (Behind a value read after the barrier: the compiler takes the timer before it.)
+    if (ht == 0 && go) st.timeline[4 * s + 3] = gtimer();
     if constexpr (!K::EARLY) {
       if (go) {
         store_leaf<K, LD>(z, sV, SV, lane, hw);
@@ -1059,10 +1060,7 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
     {
       // ---- factor the leaf
       if (top) {
-        if (lane == 0) {
-          st.timeline[4 * s + 0] = gtimer();
-          st.timeline[4 * s + 1] = st.timeline[4 * s + 0];
-        }
+        if (lane == 0) st.timeline[4 * s + 0] = gtimer();
         factor_top<K>(a, sm, w, gq, t, st.tau + (long long)z.f.k * n + z.f.j0);
       } else {
         factor_rows<K>(a, sm, w, ab8, nb, gq, t, warp);
@@ -1113,6 +1111,7 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
       if constexpr (K::BULK) tc::fence_proxy_async_smem();  // V is stored to global memory by bulk copies
       if constexpr (K::EARLY) bar_v_arrive<K::CT>();
     }
+    if (warp == 0 && lane == 0) st.timeline[4 * s + 1] = gtimer();
     bar_ready<K::THREADS>();
     if (!sm.ok[s & 1]) {
       bar_done<K::THREADS>();

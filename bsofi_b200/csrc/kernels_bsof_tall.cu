@@ -291,7 +291,6 @@ __global__ void __launch_bounds__(BT, 1) bsof_tall_kernel(BsofGeom g, BsofState 
       tile_range(g, f.m, f.t, lo, hi);
       if (tid == 0) st.timeline[4 * s + 0] = gtimer();
       if (!own && !block_wait_geq(st, st.cnt + tile_id(g, f.m, f.t), hi - lo, &sm.flag)) return;
-      if (tid == 0) st.timeline[4 * s + 1] = gtimer();
       const int mrows = 2 * g.n - f.j0;
       long long ldp;
       double* P = mat_ptr(g, st, (long long)f.k * g.n + f.j0, f.m, f.t * g.NB, ldp);
@@ -333,6 +332,7 @@ __global__ void __launch_bounds__(BT, 1) bsof_tall_kernel(BsofGeom g, BsofState 
         Tout[e] = (rr < f.w && cc < f.w) ? sm.T[rr][cc] : 0.0;
       }
       __syncthreads();
+      if (tid == 0) st.timeline[4 * s + 1] = gtimer();
       // Apply leaf s to the tile of leaf s+1.  That is the tile's last update
       // and only this CTA reads the tile next, so it is not published; the
       // leaf itself (reflectors and T) is published after the update, with one

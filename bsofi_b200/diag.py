@@ -11,7 +11,8 @@ bsof-timeline inverts a seeded Hubbard matrix (a random p-cyclic one when n is
 not a square) with bsofi_device_invert and prints, for the last run, the BSOF
 chain length and the per-leaf phases recorded by the persistent BSOF kernel's
 critical CTA (bsofi_device_bsof_timeline: globaltimer stamps at leaf start,
-next-tile update start and leaf done).  invert times REPS
+leaf factored, next-tile update start and leaf done; the wait is the time
+between the second and the third, in which the next tile arrives).  invert times REPS
 device-resident inversions of the Hubbard matrix (U = 4 unless given) with the
 size's launch plan and prints the fastest with its TFLOP/s, the BSOI time
 (CUDA events around its launches) and the BSOF chain.
@@ -66,22 +67,22 @@ def bsof_timeline(n, L, reps=3):
             "invert_ms": e0.elapsed_time(e1),
             "chain_ms": (t[-1, 2] - t[0, 0]) / 1e6,
             "leaves": S,
-            "wait_tile_us": (t[:, 1] - t[:, 0]).mean() / 1e3,
-            "factor_us": (has[:, 3] - has[:, 1]).mean() / 1e3,
+            "wait_tile_us": (has[:, 3] - has[:, 1]).mean() / 1e3,
+            "factor_us": (has[:, 1] - has[:, 0]).mean() / 1e3,
             "update_publish_us": (has[:, 2] - has[:, 3]).mean() / 1e3,
             "to_next_leaf_us": (t[1:, 0] - t[:-1, 2]).mean() / 1e3,
         }
-        wait = (t[:, 1] - t[:, 0]) / 1e3
+        wait = (has[:, 3] - has[:, 1]) / 1e3  # of leaf s, for the tile of leaf s+1
         nl = (n + (16 if n <= 256 else 8) - 1) // (16 if n <= 256 else 8)
-        first = np.arange(S) % nl == 0  # the first leaf of each regular panel
-        first[(L - 2) * nl:] = False
+        first = np.arange(1, S) % nl == 0  # for the first leaf of each regular panel
+        first[max(0, (L - 2) * nl - 1):] = False
         out.update({
             "wait_total_ms": wait.sum() / 1e3,
             "wait_first_leaf_ms": wait[first].sum() / 1e3,
             "wait_p50_us": float(np.percentile(wait, 50)),
             "wait_p90_us": float(np.percentile(wait, 90)),
             "wait_max_us": float(wait.max()),
-            "factor_total_ms": (has[:, 3] - has[:, 1]).sum() / 1e6,
+            "factor_total_ms": (has[:, 1] - has[:, 0]).sum() / 1e6,
             "update_total_ms": (has[:, 2] - has[:, 3]).sum() / 1e6,
         })
     return out
@@ -370,7 +371,7 @@ def main(argv):
         r = bsof_timeline(n, L, reps)
         print("n %d L %d: invert %.3f ms, BSOF chain %.3f ms over %d leaves" %
               (n, L, r["invert_ms"], r["chain_ms"], r["leaves"]))
-        print("per leaf: wait for tile %.2f us, factor (tile ready -> next-tile update) %.2f us, "
+        print("per leaf: wait for tile %.2f us, factor %.2f us, "
               "next-tile update + publish %.2f us, publish -> next leaf %.2f us" %
               (r["wait_tile_us"], r["factor_us"], r["update_publish_us"], r["to_next_leaf_us"]))
         print("totals: wait %.2f ms (first leaf of a panel %.2f ms; per leaf p50 %.2f us, p90 %.2f us,"

@@ -470,8 +470,8 @@ int bsofi_device_timing_read(double *ms, long long *launches);
 
 /* Diagnostics (no reference counterpart): the BSOF timeline of the last
  * factorization that used `dwork` -- four globaltimer stamps (ns) per leaf
- * from the CTA that runs the critical chain: leaf start (twice), leaf done,
- * next-tile update start.  Copies up to max_leaves leaves to host
+ * from the CTA that runs the critical chain: leaf start, leaf factored, leaf
+ * done, next tile there and its update started (undefined where there is none).  Copies up to max_leaves leaves to host
  * and returns the number copied.  set_bsof_workers sets the number of worker
  * CTAs of the persistent BSOF kernel (default 32) for this process. */
 int bsofi_device_bsof_timeline(int n, int L, int ldda, void *dwork, unsigned long long *host,
