@@ -365,6 +365,11 @@ def main(argv):
         if a.startswith("--workers="):
             _lib.load().bsofi_device_set_bsof_workers(int(a.split("=", 1)[1]))
             argv = [x for x in argv if x != a]
+    # --factor-warps=W: accepted, without effect (an earlier chain kernel's choice).
+    for a in list(argv):
+        if a.startswith("--factor-warps="):
+            _lib.load().bsofi_device_set_bsof_factor_warps(int(a.split("=", 1)[1]))
+            argv = [x for x in argv if x != a]
     if len(argv) >= 3 and argv[0] == "bsof-timeline":
         n, L = int(argv[1]), int(argv[2])
         reps = int(argv[3]) if len(argv) > 3 else 3
