@@ -869,11 +869,14 @@ BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const dou
     const int gq = lane >> 2, t = lane & 3;
     for (int s = st.s_begin; s < st.s_end; s++) {
       const Leaf f = sm.step[s & 1].f;
+      // (Stamps by this warp where they can be: the chain does not wait for it.)
+      if (lane == 0) st.timeline[4 * s + 0] = gtimer();
       double T[K::CN][2 * K::CN] = {};
       for (int I = 0; I <= f.w; I++) {
         bar_col<K::CT>();
         if (I > 0) t_column<K::CN>(T, sm.vtv[(I - 1) & 1], I - 1, gq, t);
       }
+      const unsigned long long factored = gtimer();
       double* Tout = st.T + ((long long)f.k * st.maxleaves + f.l) * 256;
 #pragma unroll
       for (int r = 0; r < K::CN; r++)
@@ -883,6 +886,7 @@ BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const dou
           sm.T[i][j] = T[r][q];
           Tout[i + 16 * j] = T[r][q];
         }
+      if (lane == 0) st.timeline[4 * s + 1] = factored;
       if constexpr (K::EARLY) {
         bar_ready_arrive<K::THREADS>();
         bar_v<K::CT>();
@@ -998,8 +1002,9 @@ BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const dou
     }
     bar_ready<K::THREADS>();
     const bool go = ok != 0;
-    // (Behind a value read after the barrier: the compiler takes the timer before it.)
-    if (ht == 0 && go) st.timeline[4 * s + 3] = gtimer();
+    // (Behind a value read after the barrier, or the compiler takes the timer before it;
+    // not by the warp that stores and publishes the leaf.)
+    if (ht == 32 && go) st.timeline[4 * s + 3] = gtimer();
     if constexpr (!K::EARLY) {
       if (go) {
         store_leaf<K, LD>(z, sV, SV, lane, hw);
@@ -1060,7 +1065,6 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
     {
       // ---- factor the leaf
       if (top) {
-        if (lane == 0) st.timeline[4 * s + 0] = gtimer();
         factor_top<K>(a, sm, w, gq, t, st.tau + (long long)z.f.k * n + z.f.j0);
       } else {
         factor_rows<K>(a, sm, w, ab8, nb, gq, t, warp);
@@ -1111,7 +1115,6 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
       if constexpr (K::BULK) tc::fence_proxy_async_smem();  // V is stored to global memory by bulk copies
       if constexpr (K::EARLY) bar_v_arrive<K::CT>();
     }
-    if (warp == 0 && lane == 0) st.timeline[4 * s + 1] = gtimer();
     bar_ready<K::THREADS>();
     if (!sm.ok[s & 1]) {
       bar_done<K::THREADS>();
