@@ -83,9 +83,6 @@ struct ChainCfg {
   // Loads a lane and column in flight where unaligned columns are copied by plain loads
   // (16-wide forms: their chain does not wait for them; the 8-wide ones use spans).
   static constexpr int LOADS = ROWS_WORK <= 128 ? 4 : (ROWS_WORK <= 256 ? 8 : 16);
-  // V as the operand of W = V^T C comes from the registers that factored it,
-  // or, where V and C do not fit in registers together, from shared memory.
-  static constexpr bool VREG = NI * CN <= 23;
   // EARLY: a leaf is published when V is in shared memory, not when the next tile
   // is, so that the workers' answer may take a chain step longer.  Where the chain
   // waits for them, an inversion at n = 576, p = 12 went from 19.6 to 17.6 ms and at
@@ -1024,6 +1021,7 @@ template <class K>
 BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV, double* part,
                              double* sC, int SV, ChainSmem<K::MW>& sm) {
   constexpr int FW = K::FW, NI = K::NI, MW = K::MW, MT = K::MT, CN = K::CN;
+  static_assert(NI * CN <= 23, "V and C in registers");
   // (The shuffle tells the compiler that the warp index is uniform.)
   const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int gq = lane >> 2, t = lane & 3, gc = col_of(gq);
@@ -1121,9 +1119,10 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
       return;
     }
     if (next) {
-      // ---- leaf s on the tile of leaf s+1.  That is the tile's last update
-      // and only this CTA reads the tile next, so it stays in registers; its
-      // rows above the next leaf are final and go to global memory.
+      // ---- leaf s on the tile of leaf s+1, V from the registers that factored
+      // it.  That is the tile's last update and only this CTA reads the tile
+      // next, so it stays in registers; its rows above the next leaf are final
+      // and go to global memory.
       double c[NI][CN][2];
       double acc[CN][2 * CN] = {};
       const bool vec = pair_aligned(C, ldc);
@@ -1150,24 +1149,10 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
             c[i][cs][1] = v.y;
           }
         }
-        if constexpr (K::VREG) {
 #pragma unroll
-          for (int i = ia; i < ie; i++)
+        for (int i = ia; i < ie; i++)
 #pragma unroll
-            for (int jt = 0; jt < CN; jt++) mma_w<CN>(acc[jt], c[i], a[i][jt][0], a[i][jt][1]);
-        }
-      }
-      if constexpr (!K::VREG) {
-#pragma unroll
-        for (int i = 0; i < NI; i++) {
-          const int b = bb + i * bs, r = 8 * b + 2 * t;
-          if (b < blo || b >= bhi) continue;
-#pragma unroll
-          for (int jt = 0; jt < CN; jt++) {
-            const double2 v = *reinterpret_cast<const double2*>(sV + sidx(r, gc + 8 * jt, SV));
-            mma_w<CN>(acc[jt], c[i], v.x, v.y);
-          }
-        }
+          for (int jt = 0; jt < CN; jt++) mma_w<CN>(acc[jt], c[i], a[i][jt][0], a[i][jt][1]);
       }
       double fr[CN][2 * CN];
       reduce_w<MW, CN>(acc, fr, part, sm, gq, t, warp);

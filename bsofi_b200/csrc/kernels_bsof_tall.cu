@@ -45,7 +45,6 @@ struct Smem {
   double W[NB][NB + 1];
   int flag;
   int task;
-  int pflag;  // next-tile prefetch of the panel CTA succeeded
 };
 
 // T(0:I, I) = -tau_I T(0:I,0:I) g_I (LAPACK dlarft), run by one warp one
@@ -279,18 +278,11 @@ __global__ void __launch_bounds__(BT, 1) bsof_tall_kernel(BsofGeom g, BsofState 
 
   if (blockIdx.x == 0) {
     // ---------------------------------------------------------- panel chain
-    // own: this CTA applied the last update to the current leaf's tile, so it
-    // needs no wait (shared barriers order its own global writes).  A launch
-    // that continues at s_begin > 0 starts owning its first tile: the earlier
-    // launch, complete before this one starts, applied that tile's last
-    // update from its panel CTA, which is never counted.
-    bool own = st.s_begin > 0;
+    // The first leaf's tile has no update to wait for, and this CTA makes the last
+    // one of every other leaf's (shared barriers order its own global writes).
     for (int s = st.s_begin; s < st.s_end; s++) {
       const Leaf f = leaf_of(g, s);
-      int lo, hi;
-      tile_range(g, f.m, f.t, lo, hi);
       if (tid == 0) st.timeline[4 * s + 0] = gtimer();
-      if (!own && !block_wait_geq(st, st.cnt + tile_id(g, f.m, f.t), hi - lo, &sm.flag)) return;
       const int mrows = 2 * g.n - f.j0;
       long long ldp;
       double* P = mat_ptr(g, st, (long long)f.k * g.n + f.j0, f.m, f.t * g.NB, ldp);
@@ -347,7 +339,6 @@ __global__ void __launch_bounds__(BT, 1) bsof_tall_kernel(BsofGeom g, BsofState 
         red_release_add(st.factored + s, 1);
         st.timeline[4 * s + 2] = gtimer();
       }
-      own = next;
     }
     return;
   }
