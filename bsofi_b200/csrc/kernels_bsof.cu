@@ -866,13 +866,13 @@ BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const dou
     const int gq = lane >> 2, t = lane & 3;
     for (int s = st.s_begin; s < st.s_end; s++) {
       const Leaf f = sm.step[s & 1].f;
-      // (Stamps by this warp where they can be: the chain does not wait for it.)
-      if (lane == 0) st.timeline[4 * s + 0] = gtimer();
       double T[K::CN][2 * K::CN] = {};
       for (int I = 0; I <= f.w; I++) {
         bar_col<K::CT>();
         if (I > 0) t_column<K::CN>(T, sm.vtv[(I - 1) & 1], I - 1, gq, t);
       }
+      // (Stamps by this warp where they can be: the chain does not wait for it.  The
+      // third one by a warp that stores the leaf took n = 255, p = 12 from 4.69 to 4.82 ms.)
       const unsigned long long factored = gtimer();
       double* Tout = st.T + ((long long)f.k * st.maxleaves + f.l) * 256;
 #pragma unroll
@@ -895,6 +895,8 @@ BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const dou
         }
       } else {
         bar_ready<K::THREADS>();
+        // (Behind a value read after the barrier, or the compiler takes the timer before it.)
+        if (lane == 0 && sm.ok[s & 1]) st.timeline[4 * s + 3] = gtimer();
       }
       if (lane == 0 && s + 1 < st.s_end) sm.step[(s + 1) & 1] = chain_step(g, st, s + 1);
       bar_done<K::THREADS>();
@@ -999,9 +1001,7 @@ BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const dou
     }
     bar_ready<K::THREADS>();
     const bool go = ok != 0;
-    // (Behind a value read after the barrier, or the compiler takes the timer before it;
-    // not by the warp that stores and publishes the leaf.)
-    if (ht == 32 && go) st.timeline[4 * s + 3] = gtimer();
+    if (K::EARLY && ht == 0 && go) st.timeline[4 * s + 3] = gtimer();
     if constexpr (!K::EARLY) {
       if (go) {
         store_leaf<K, LD>(z, sV, SV, lane, hw);
@@ -1063,6 +1063,13 @@ BSOFI_DEVINL void chain_main(const BsofGeom& g, const BsofState& st, double* sV,
     {
       // ---- factor the leaf
       if (top) {
+        // (The second store, which the T warp's follows, only keeps an order of
+        // instructions that measured faster: n = 144, p = 20 3.51 ms against 3.54.)
+        if (lane == 0) {
+          const unsigned long long now = gtimer();
+          st.timeline[4 * s + 0] = now;
+          st.timeline[4 * s + 1] = now;
+        }
         factor_top<K>(a, sm, w, gq, t, st.tau + (long long)z.f.k * n + z.f.j0);
       } else {
         factor_rows<K>(a, sm, w, ab8, nb, gq, t, warp);

@@ -62,8 +62,6 @@ def bsof_timeline(n, L, reps=3):
         if cnt != S:
             raise RuntimeError("timeline holds %d leaves, expected %d" % (cnt, S))
         t = buf.reshape(S, 4).astype(np.int64)
-        # A leaf starts when the one before is done (two warps take these stamps).
-        t[1:, 0] = np.maximum(t[1:, 0], t[:-1, 2])
         has = t[:-1]
         out = {
             "invert_ms": e0.elapsed_time(e1),
