@@ -12,10 +12,12 @@
 // eight warps at n = 100), instruction issue and the barrier of every chunk
 // for the 8-row bands of small problems.  Measured (BSOI alone, us; before:
 // one launch of 64 x 64 tiles per step, or one persistent launch of them):
-// n = 16, p = 8 75 -> 18; n = 64, p = 16 252 -> 61; n = 64, p = 100 1457 ->
-// 867; n = 100, p = 32 838 -> 451; n = 100, p = 64 1570 -> 1450; n = 128,
-// p = 20 564 -> 337; n = 128, p = 60 even (2016).  Above n = 128 the carry and
-// the stages leave no room for tall bands.
+// n = 16, p = 8 75 -> 18; n = 64, p = 16 254 -> 61; n = 64, p = 100 1472 ->
+// 870; n = 100, p = 32 837 -> 451; n = 100, p = 64 1565 -> 1456; n = 128,
+// p = 20 564 -> 342; n = 128, p = 40 1027 -> 977.  Above n = 112 the carry and the
+// stages leave room for 48 rows only, and n = 128, p = 55 takes longer than before
+// (1690 -> 1948): pipeline.cu ends the bands before that.  Above n = 128 there is no
+// room for tall bands at all.
 //
 // Bands are cut on the host: rows of X below the diagonal block are zero in
 // segment X(:,k), so a row near the bottom costs half of one at the top.

@@ -129,17 +129,30 @@ thread_local bool g_wait_test = false;
 
 // Whether BSOI runs as one launch of row bands (kernels_bsoi_band.cu) and
 // BSTRI's recurrence as one of column bands (kernels_bstri_band.cu): blocks of
-// at most 128 with row bands of at most 64 rows, one per SM, where the plan's
-// knob is the size's default (a tuned plan that chose another form keeps it).
-// In pipelined batches only where the launches are short (a long one would
+// at most 128 with one row band per SM, of at most 64 rows (48 above n = 112), where
+// the plan's knob is the size's default (a tuned plan that chose another form keeps
+// it).  In pipelined batches only where the launches are short (a long one would
 // keep the next chains' launches waiting).
 bool band_size(int n, int L) {
   if (g_nonpersistent && n * L > 2400) return false;
   return bsoi_band_fits(n, L);
 }
 
+// BSOI's bands end earlier where their output tiles fill the warps badly and their
+// rows the SM: inversions in us, BSOI by tiles -> by bands: n = 121, p = 49
+// 7473 -> 7342, 52 7780 -> 7861; n = 128, p = 42 5448 -> 5418, 45 5895 -> 5892, 51
+// 6824 -> 6976; n = 96, p = 90 8942 -> 8987, 95 9570 -> 9702; n = 72, p = 126 9930 -> 9700.
+// Up to n = 64 and for n = 97..112 (four tiles of 64 columns for three and a half)
+// bands are the faster ones to the end (BSOI's steps alone: n = 64, p = 146 2230 -> 1733,
+// n = 100, p = 94 3329 -> 3118).
+bool bsoi_band_pays(int n, int L) {
+  const long long N = (long long)n * L;
+  if (n > 112) return N <= 5800;
+  return n <= 64 || n > 96 || N <= 9000;
+}
+
 bool use_bsoi_band(int n, int L) {
-  if (g_wait_test || !band_size(n, L)) return false;
+  if (g_wait_test || !bsoi_band_pays(n, L) || !band_size(n, L)) return false;
   const Plan p = stored_plan(n, L), d = default_plan(n, L);
   return p.bsoi == d.bsoi && (p.bsoi == 1 || p.bsoi == 5);
 }
