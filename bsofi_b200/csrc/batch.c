@@ -134,14 +134,16 @@ void bsofi_device_set_batch_pipelined(int on) { flag_set(&g_pipelined, on ? 1 : 
  * 48.6 -> 34.6, 7 30.0 -> 18.5, 4 44.0 -> 32.4.  The line at 12 in flight: 13 and
  * 16 instances took 79.8 and 67.1 with 10 for all, 85.1 and 70.6 with 14 and 12
  * for the large ones; 12 instances 36.8 with 10 for all, 31.2 with 16 and 8.
- * Where instances queue behind 6 to 12 streams the GPU is full of their products
- * and the few chains' 25 to 33 CTAs keep SMs from them: 8, and 12 for the large
- * blocks.  On 8 streams, with 12 and 16 -> 8 and 12: 48 instances 138.3 -> 133.8, 20
- * 56.0 -> 53.7, 17 48.8 -> 45.8, 14 36.3 -> 34.4, 12 of n <= 121 20.8 -> 17.7, 12 of
- * all sizes 55.9 -> 54.4 and (a single large one at the end) 25.3 -> 32.7.  Four
- * chains of 33 CTAs fit the GPU, so 4 and 5 streams do so only where the queue is
- * deep: 48 instances on 4 streams 143.8 -> 138.1, 36 150.4 -> 150.2, but 20
- * 37.4 with 16, 39.9 with 8 and 12. */
+ * Where instances queue behind 6 to 12 streams, the products of the others want the
+ * SMs too: 8 for small blocks, and 10 for large ones (21 CTAs, seven chains at
+ * once) where every slot has two or more to run; in a shorter queue the last large
+ * instance runs alone and keeps 16.  On 8 streams, with 12 below n = 180 and 16 from
+ * there on -> with this rule: 48 instances 138.1 -> 132.2, 20 55.8 -> 53.2, 17 48.9 ->
+ * 45.9, 16 of n = 256, p = 32 108.7 -> 107.9 (111.0 with 12), 16 of n = 144 41.3 -> 38.6,
+ * 32 of n <= 64 11.2 -> 9.2; 12 of n <= 121 20.8 -> 17.7, 12 of all sizes 25.4 -> 23.6;
+ * on 6 streams 64 instances 173.7 -> 156.2.  Four chains of 33 CTAs fit the GPU, so 4 and
+ * 5 streams take fewer only where the queue is long: 48 instances on 4 streams 143.8 ->
+ * 137.9, 36 150.2 -> 149.9, but 20 37.4 with 16, 39.9 with 8 and 12. */
 static int g_batch_workers = 0;
 void bsofi_device_set_batch_workers(int w) { flag_set(&g_batch_workers, w < 0 ? 0 : w); }
 int bsofi_batch_workers(int n, int count, int in_flight) {
@@ -149,8 +151,11 @@ int bsofi_batch_workers(int n, int count, int in_flight) {
   if (w > 0) return w;
   if (n > 256) return 24;
   if (in_flight > 12) return 10;
-  if (in_flight >= 6 ? count > in_flight : in_flight >= 4 && count > 8 * in_flight)
-    return n >= 224 ? 12 : 8;
+  if (in_flight >= 6 && count > in_flight) {
+    const int deep = count >= 2 * in_flight;
+    return n < (deep ? 144 : 180) ? 8 : (deep ? 10 : 16);
+  }
+  if (in_flight >= 4 && count > 8 * in_flight) return n >= 224 ? 12 : 8;
   return n >= 180 || in_flight < 6 ? 16 : 96 / in_flight;
 }
 

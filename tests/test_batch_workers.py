@@ -11,13 +11,16 @@ def test_server_request(n, workers):
     assert _lib.load().bsofi_batch_workers_for(n) == workers
 
 
-@pytest.mark.parametrize("count,streams", [(9, 8), (12, 8), (17, 8), (48, 8), (7, 6), (13, 12),
-                                           (48, 4), (41, 5)])
-def test_batch_behind_few_streams(count, streams):
-    """Instances that queue fill the GPU with their products: few workers for the chains."""
+@pytest.mark.parametrize("count,streams,workers", [
+    (9, 8, [8, 8, 8, 16, 16, 24]), (15, 8, [8, 8, 8, 16, 16, 24]), (7, 6, [8, 8, 8, 16, 16, 24]),
+    (13, 12, [8, 8, 8, 16, 16, 24]),  # a short queue: the last large instance runs alone
+    (16, 8, [8, 10, 10, 10, 10, 24]), (48, 8, [8, 10, 10, 10, 10, 24]),
+    (12, 6, [8, 10, 10, 10, 10, 24]), (24, 12, [8, 10, 10, 10, 10, 24]),
+    (48, 4, [8, 8, 8, 8, 12, 24]), (41, 5, [8, 8, 8, 8, 12, 24])])
+def test_batch_behind_few_streams(count, streams, workers):
+    """Instances that queue want SMs for their products: fewer for the chains."""
     lib = _lib.load()
-    assert [lib.bsofi_batch_workers(n, count, streams) for n in (64, 223, 224, 256, 257)] == \
-        [8, 8, 12, 12, 24]
+    assert [lib.bsofi_batch_workers(n, count, streams) for n in (143, 144, 179, 180, 256, 257)] == workers
 
 
 @pytest.mark.parametrize("count,streams,small,large", [(1, 1, 16, 16), (5, 5, 16, 16), (6, 6, 16, 16),
