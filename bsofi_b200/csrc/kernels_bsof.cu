@@ -86,8 +86,8 @@ struct ChainCfg {
   // EARLY: a leaf is published when V is in shared memory, not when the next tile
   // is, so that the workers' answer may take a chain step longer.  Where the chain
   // waits for them, an inversion at n = 576, p = 12 went from 19.6 to 17.6 ms and at
-  // n = 529 from 20.3 to 18.0; 16-wide leaves do not wait, and the extra barrier
-  // costs (n = 256, p = 32 11.65 -> 11.82, n = 400, p = 16 12.9 -> 13.3).
+  // n = 529 from 20.3 to 18.0 (it still waits there, 2 of 11 us a leaf at n = 576); 16-wide
+  // leaves do not wait, and the extra barrier costs (n = 256, p = 32 11.65 -> 11.82).
   static constexpr bool EARLY = CN == 1;
   // With 12 warps a thread gets 168 registers at launch; the helper warpgroup
   // gives most of its own to the two that compute
@@ -1759,9 +1759,11 @@ using Chain64 = ChainCfg<3, 5, 4>;
 using Chain128 = ChainCfg<7, 5, 4>;
 using Chain256 = ChainCfg<7, 9, 8>;
 using Chain416 = ChainCfg<7, 15, 13, 1>;
-using FormQ400 = ChainCfg<7, 14, 13>;
+// (The next two spill 260 and 340 bytes a thread: the leaf takes 84 and 92 registers, the
+// pivot column or the next tile beside it as many again.)
 using Chain592 = ChainCfg<7, 21, 19, 1>;
 using Chain640 = ChainCfg<7, 23, 20, 1>;
+using FormQ400 = ChainCfg<7, 14, 13>;
 using FormQ640 = ChainCfg<7, 23, 20>;
 
 // Leaf width.  Wide leaves halve the publications and updates, but a column step's
