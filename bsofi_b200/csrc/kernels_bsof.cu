@@ -895,8 +895,9 @@ BSOFI_DEVINL void chain_helper(const BsofGeom& g, const BsofState& st, const dou
         }
       } else {
         bar_ready<K::THREADS>();
-        // (Behind a value read after the barrier, or the compiler takes the timer before it.)
-        if (lane == 0 && sm.ok[s & 1]) st.timeline[4 * s + 3] = gtimer();
+        // (Behind a value read after the barrier, or the compiler takes the timer before it;
+        // not by the lane that works out the next step: n = 16, p = 40 0.468 -> 0.466 ms.)
+        if (lane == 16 && sm.ok[s & 1]) st.timeline[4 * s + 3] = gtimer();
       }
       if (lane == 0 && s + 1 < st.s_end) sm.step[(s + 1) & 1] = chain_step(g, st, s + 1);
       bar_done<K::THREADS>();
